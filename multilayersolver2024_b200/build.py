@@ -46,7 +46,7 @@ def build(verbose: bool = False, force: bool = False) -> Path:
     deps = sources + sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h")) + [INCLUDE / "mlxpbd.h"]
     if force or _stale(LIB, deps):
         tmp = LIB.with_suffix(".so.tmp")
-        _run([_nvcc(), *NVCC_FLAGS, "-shared", "-o", tmp, *sources], verbose)
+        _run([_nvcc(), *NVCC_FLAGS, "--threads", "0", "-shared", "-o", tmp, *sources], verbose)
         os.replace(tmp, LIB)
     mex_src = [MEX / "mexLayerSolve3D.cpp", MEX / "mxshim.cpp"]
     if all(p.exists() for p in mex_src) and (force or _stale(MEXLIB, mex_src + [MEX / "mex.h", LIB])):

@@ -157,7 +157,7 @@ __global__ void k_contact_mask(const R4<R>* __restrict__ x0, int N, const Obstac
 
 // Order-preserving compaction, pass 1: per-block counts of the selected
 // vertices (bit `f` of the mask, or any bit when f < 0).
-__global__ void __launch_bounds__(256) k_compact_count(const unsigned* __restrict__ mask, int N, int f,
+static __global__ void __launch_bounds__(256) k_compact_count(const unsigned* __restrict__ mask, int N, int f,
                                                        int* __restrict__ block_counts) {
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   const bool sel = v < N && (f < 0 ? mask[v] != 0 : ((mask[v] >> f) & 1u));
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(256) k_compact_count(const unsigned* __restric
 // Pass 2 (one CTA of 1024 threads): exclusive prefix sum of the block
 // counts, in place, starting at *base (0 when base is NULL); base + the sum
 // lands in *total.
-__global__ void __launch_bounds__(1024) k_compact_scan(int* __restrict__ block_counts, int nblocks,
+static __global__ void __launch_bounds__(1024) k_compact_scan(int* __restrict__ block_counts, int nblocks,
                                                        const int* __restrict__ base_ptr, int* __restrict__ total) {
   __shared__ int part[1024];
   const int base = base_ptr ? *base_ptr : 0;
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(1024) k_compact_scan(int* __restrict__ block_c
 
 // Pass 3: every selected vertex writes its rank.  out_vert[rank] = v and
 // (optionally) rank_of[v] = rank, -1 for the others.
-__global__ void __launch_bounds__(256) k_compact_scatter(const unsigned* __restrict__ mask, int N, int f,
+static __global__ void __launch_bounds__(256) k_compact_scatter(const unsigned* __restrict__ mask, int N, int f,
                                                          const int* __restrict__ block_offsets,
                                                          int* __restrict__ out_vert, int* __restrict__ rank_of) {
   __shared__ int warp_tot[8];
@@ -296,7 +296,7 @@ __global__ void k_contact_velocity(const DevContacts dc, const R4<R>* __restrict
 
 // Length of each finder's contact list: the vertices whose mask has bit f
 // (integer atomics, so the counts are exact).  `counts` is zeroed before.
-__global__ void __launch_bounds__(256) k_obstacle_counts(const unsigned* __restrict__ mask, int N, int nobs,
+static __global__ void __launch_bounds__(256) k_obstacle_counts(const unsigned* __restrict__ mask, int N, int nobs,
                                                          int* __restrict__ counts) {
   __shared__ int s[32];
   if (threadIdx.x < 32) s[threadIdx.x] = 0;
@@ -361,11 +361,11 @@ __global__ void __launch_bounds__(256) k_contact_residual_partials(const DevCont
 // contact_coloring, per step: the contact vertices bucketed by their colour
 // phase (counts, offsets, scatter).  The order inside a bucket is free: a
 // bucket holds distinct vertices, each projected by one thread.
-__global__ void k_cc_hist(const DevContacts dc, int* __restrict__ hist) {
+static __global__ void k_cc_hist(const DevContacts dc, int* __restrict__ hist) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < *dc.count) atomicAdd(hist + dc.vcc[dc.verts[i]], 1);
 }
-__global__ void k_cc_offsets(const int* __restrict__ hist, int nb, int* __restrict__ off, int* __restrict__ cur) {
+static __global__ void k_cc_offsets(const int* __restrict__ hist, int nb, int* __restrict__ off, int* __restrict__ cur) {
   if (blockIdx.x || threadIdx.x) return;
   int run = 0;
   for (int c = 0; c < nb; ++c) {
@@ -375,7 +375,7 @@ __global__ void k_cc_offsets(const int* __restrict__ hist, int nb, int* __restri
   }
   off[nb] = run;
 }
-__global__ void k_cc_scatter(const DevContacts dc, int* __restrict__ cur, int* __restrict__ bucket) {
+static __global__ void k_cc_scatter(const DevContacts dc, int* __restrict__ cur, int* __restrict__ bucket) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < *dc.count) {
     const int v = dc.verts[i];

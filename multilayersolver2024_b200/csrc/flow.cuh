@@ -1,0 +1,180 @@
+// flow.cuh -- the projectGS loop of one layer as a dataflow over vertex
+// versions, records pushed through (distributed) shared memory.
+//
+// Every tet reads and writes each of its four vertices once per sweep, so the
+// Gauss-Seidel order of the colours (xpbdLayer3D.m:357-378) is one chain per
+// vertex: the tets at a vertex in colour order, each reading the record the
+// one before it wrote.  Here a tet writes its four corners straight into the
+// shared memory of the CTA that projects each vertex's next tet, and every
+// store counts on an mbarrier of the chunk of 32 tets that the next tet
+// belongs to: a store and an arrive inside the CTA, st.async and its bytes
+// across CTAs.  A warp sleeps on its chunk's mbarrier until all of the chunk's
+// records are there: no barrier, fence, poll or launch separates the colours,
+// and colours overlap wherever the vertices allow.
+//
+// Layout.  The mesh's elements are cut into G groups of whole connected
+// components, one thread-block cluster of CS CTAs each, and a group's
+// elements into CS parts, one per CTA rank.  A CTA has one slot (x, y, z, 1/m)
+// per vertex its tets touch.  A vertex's versions form one chain, so a slot is
+// never overwritten before it was read.  Per layer and corner the host fixes
+// the slot that is read, the rank, slot and chunk of the vertex's next tet and
+// the corner word (below).  A vertex's first tet of the first iteration reads
+// the position array and its last tet of the last iteration writes it, so a
+// launch begins and ends there.
+//
+// A CTA's tets are cut into chunks of at most 32 of one colour, in colour
+// order; chunk j is warp j mod nw's in every iteration, so a tet's
+// multipliers stay with one thread.  The CTAs of a cluster are co-scheduled
+// and every warp works in order, so the first unfinished chunk can always
+// run.  A chunk's barrier is armed for iteration it + 1 before iteration it's
+// results leave the warp, and whatever arrives for it + 1 depends on those.
+// A wait that lasts kWaitNs sets the error flag and ends the launch.
+//
+// What bounds it: a vertex's chain, one projection (~1,200 cycles for a
+// Neo-Hookean tet), its stores' way to the next CTA and the wake-up per tet,
+// ~0.9 us per colour on meshes whose chunks leave the SMs idle; above ~100
+// chunks per CTA the warps share the SM (~250 cycles per chunk).  A colour
+// launch costs ~1.9 us whatever its size.  Per sweep (B200, Neo-Hookean FP32,
+// this path / colour launches): 27,648 tets on 16 CTAs 29 / 58 us, 98,304
+// tets 41 / 58 us, 64 scenes of 866 k tets 53 / 95 us.  Polling the records'
+// versions instead of mbarriers measured 33 us on the 27,648 tets (the polls
+// take the shared-memory pipe from the projections), st.async inside the CTA
+// too 45 us on the 98,304 (it goes out to the network and back), bulk copies
+// of the rest data into shared memory no gain.
+//
+// The per-vertex phases of an iteration join the chain: the contacts of a
+// vertex run where their phase falls between two of its tets (before the tet
+// that follows, or after the last), the pinned DOFs after the last.
+#pragma once
+
+#include "cluster.cuh"
+#include "common.cuh"
+#include "contacts.cuh"
+#include "persistent.cuh"
+#include "tet_kernels.cuh"
+
+namespace mlx {
+
+template <typename R> __host__ __device__ constexpr int flow_threads() { return sizeof(R) == 4 ? 512 : 256; }
+// corner word, marks of the vertex at this tet: first and last of the layer's
+// tets at the vertex (in colour order), pinned DOFs, contacts before this tet
+// or after it (contact colouring), no body
+constexpr unsigned kFlowFirst = 1, kFlowLast = 2, kFlowPinned = 4, kFlowBefore = 8, kFlowAfter = 16, kFlowFree = 32;
+constexpr int kFlowMaxSlots = 1 << 14, kFlowMaxChunks = 1 << 14;
+
+// corner of a tet: x = slot it is read from | corner word << 16, y = where the
+// vertex's next tet reads it: rank << 28 | chunk << 14 | slot
+struct FlowCorner {
+  uint2 c[4];
+};
+
+template <typename R> struct FlowArgs {
+  const int* part_off;      // [G CS + 1] chunks of each part
+  // first position in the list (sorted id if no list); tets; records that
+  // other CTAs send for iteration 0; records that come from this CTA, those of
+  // them that no tet sends for iteration 0 << 16
+  const int4* chunks;
+  const int* list;          // layer's elastic tets, NULL = identity
+  const FlowCorner* corner; // [T] sorted ids
+  const int* pin_at;        // [3N] index into pin_vals or -1
+  const R* pin_vals;
+  int* error;
+  int cs, slots, iterations;
+  int pins;                 // apply the pinned DOFs at the end of every iteration
+  int after;                // contacts after the last tet: 0 none, 1 all, 2 those marked kFlowAfter
+  double h, contact_resistance;
+};
+
+__device__ __forceinline__ void flow_push(uint32_t a, uint32_t bar, float4 v) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(a),
+               "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void flow_push(uint32_t a, uint32_t bar, double4 v) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(a),
+               "d"(v.x), "d"(v.y), "r"(bar)
+               : "memory");
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(a + 16),
+               "d"(v.z), "d"(v.w), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void flow_st(uint32_t a, float4 v) {
+  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+__device__ __forceinline__ void flow_st(uint32_t a, double4 v) {
+  asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v.x), "d"(v.y) : "memory");
+  asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(a + 16), "d"(v.z), "d"(v.w) : "memory");
+}
+__device__ __forceinline__ void flow_bar_init(uint32_t bar, unsigned count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void flow_arrive(uint32_t bar, unsigned n) {
+  asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(n) : "memory");
+}
+// completes the barrier's phase once `bytes` have arrived in it
+__device__ __forceinline__ void flow_arm(uint32_t bar, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool flow_try(uint32_t bar, unsigned parity) {
+  unsigned ok;
+  asm volatile("{.reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p;}"
+               : "=r"(ok)
+               : "r"(bar), "r"(parity)
+               : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ float4 flow_ld(uint32_t a, float) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ double4 flow_ld(uint32_t a, double) {
+  double4 v;
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a) : "memory");
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.z), "=d"(v.w) : "r"(a + 16) : "memory");
+  return v;
+}
+
+// Waits (a whole warp) for the phase of a chunk's records, at most kWaitNs;
+// false when it gave up or another wait has.
+__device__ __forceinline__ bool flow_wait(uint32_t bar, unsigned parity, int* error) {
+  unsigned spins = 0;
+  unsigned long long t0 = 0;
+  while (!__all_sync(0xffffffffu, flow_try(bar, parity))) {
+    if ((++spins & 63u) != 0) continue;
+    bool over = *reinterpret_cast<volatile int*>(error) != 0;
+    const unsigned long long t = global_ns();
+    if (t0 == 0) t0 = t;
+    if (t - t0 > kWaitNs) {
+      atomicExch(error, 1);
+      over = true;
+    }
+    if (__any_sync(0xffffffffu, over)) return false;
+  }
+  return true;
+}
+
+// A vertex record in registers, for the contact projection.
+template <typename R> struct FlowPos {
+  R4<R>* p;
+  __device__ __forceinline__ R4<R> ld(int) const { return *p; }
+  __device__ __forceinline__ void st(int, R4<R> x) const { *p = x; }
+};
+
+// The device-detected elastic contacts of vertex v with record p.
+template <typename R>
+__device__ __forceinline__ void flow_contacts(const DevContacts& dc, int v, R4<R>& p, const R4<R>* __restrict__ x0,
+                                              double h, double resistance) {
+  const int i = dc.cidx[v];
+  if (i >= 0) elastic_contacts_of_vertex<R>(dc, i, FlowPos<R>{&p}, x0, h, resistance);
+}
+
+// k_flow of a precision and material (flow_fp32.cu, flow_fp64.cu); `ct`: with
+// device-detected contacts.
+const void* flow_kernel_fp32(int mat_kind, bool damp, bool ct);
+const void* flow_kernel_fp64(int mat_kind, bool damp, bool ct);
+inline const void* flow_kernel(bool fp64, int mat_kind, bool damp, bool ct) {
+  return fp64 ? flow_kernel_fp64(mat_kind, damp, ct) : flow_kernel_fp32(mat_kind, damp, ct);
+}
+
+}  // namespace mlx

@@ -42,12 +42,12 @@ int bfs(int start, const std::vector<int>& vt_off, const std::vector<int>& vt, c
   return last;
 }
 
-}  // namespace
-
-void partition_mesh(int N, int T, const int32_t* t, int parts, MeshPartition& out) {
-  out.parts = parts;
+// Breadth-first order of all vertices, component by component, each from a
+// pseudo-peripheral vertex; vt_off: offsets of the vertices' incident tets.
+void breadth_first_vertices(int N, int T, const int32_t* t, std::vector<int>& vt_off, std::vector<int>& order) {
   // vertex -> tets incidence (CSR)
-  std::vector<int> vt_off(N + 1, 0), vt(4 * (size_t)T);
+  vt_off.assign(N + 1, 0);
+  std::vector<int> vt(4 * (size_t)T);
   for (int e = 0; e < T; ++e)
     for (int k = 0; k < 4; ++k) ++vt_off[t[e + (size_t)T * k]];
   for (int v = 0; v < N; ++v) vt_off[v + 1] += vt_off[v];
@@ -57,7 +57,7 @@ void partition_mesh(int N, int T, const int32_t* t, int parts, MeshPartition& ou
       for (int k = 0; k < 4; ++k) vt[fill[t[e + (size_t)T * k] - 1]++] = e;
   }
   // breadth-first order, component by component
-  std::vector<int> order;
+  order.clear();
   order.reserve(N);
   std::vector<char> seen(N, 0), probe(N, 0);
   for (int v0 = 0; v0 < N; ++v0) {
@@ -66,6 +66,14 @@ void partition_mesh(int N, int T, const int32_t* t, int parts, MeshPartition& ou
     int far = bfs(v0, vt_off, vt, t, T, probe, tmp);
     bfs(far, vt_off, vt, t, T, seen, order);
   }
+}
+
+}  // namespace
+
+void partition_mesh(int N, int T, const int32_t* t, int parts, MeshPartition& out) {
+  out.parts = parts;
+  std::vector<int> vt_off, order;
+  breadth_first_vertices(N, T, t, vt_off, order);
   // cut into runs of equal incident-tet weight (isolated vertices weigh 1)
   long long W = 0;
   for (int v = 0; v < N; ++v) W += std::max(vt_off[v + 1] - vt_off[v], 1);
@@ -108,6 +116,21 @@ void partition_mesh(int N, int T, const int32_t* t, int parts, MeshPartition& ou
     }
     out.tpart[e] = best;
   }
+}
+
+void breadth_first_elements(int N, int T, const int32_t* t, std::vector<int>& order) {
+  std::vector<int> vt_off, verts, at(N), first(N + 1, 0);
+  breadth_first_vertices(N, T, t, vt_off, verts);
+  for (int i = 0; i < N; ++i) at[verts[i]] = i;
+  auto key = [&](int e) {
+    int k = N;
+    for (int c = 0; c < 4; ++c) k = std::min(k, at[t[e + (size_t)T * c] - 1]);
+    return k;
+  };
+  for (int e = 0; e < T; ++e) ++first[key(e) + 1];
+  for (int i = 0; i < N; ++i) first[i + 1] += first[i];
+  order.assign(T, 0);
+  for (int e = 0; e < T; ++e) order[first[key(e)]++] = e;
 }
 
 }  // namespace mlx

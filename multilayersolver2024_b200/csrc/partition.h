@@ -19,4 +19,8 @@ struct MeshPartition {
 // Splits a tet mesh (t: T x 4, column-major, 1-based) into `parts` pieces.
 void partition_mesh(int N, int T, const int32_t* t, int parts, MeshPartition& out);
 
+// Elements in breadth-first order (by their earliest corner in the order
+// partition_mesh cuts): consecutive runs are slabs of level sets.
+void breadth_first_elements(int N, int T, const int32_t* t, std::vector<int>& order);
+
 }  // namespace mlx

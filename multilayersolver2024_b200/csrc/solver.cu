@@ -17,6 +17,7 @@
 #include "persistent.cuh"
 #include "cluster.cuh"
 #include "groups.cuh"
+#include "flow.cuh"
 #include "layers_dev.cuh"
 #include "contacts.cuh"
 #include "monitor.cuh"
@@ -29,6 +30,7 @@
 #include <cub/device/device_scan.cuh>
 
 #include <algorithm>
+#include <cmath>
 #include <cstddef>
 #include <chrono>
 #include <cstdlib>
@@ -215,6 +217,15 @@ struct LayerStatic {
   int gr_one = 0;
   size_t o_goff = 0;
   std::vector<int> tile;  // block size of each colour kernel (0 = default), set by the autotuner
+  // dataflow path (flow.cuh): chunks of each part, corner words and slots
+  bool fl_ok = false;
+  int fl_chunks = 0, fl_max = 0;  // chunks, largest part's
+  bool fl_loose_pins = false;  // a pinned vertex has no elastic tet in this layer
+  bool fl_loose_free = false;  // a vertex of no body has none
+  bool fl_coloured = false;    // the corner words hold the contact phases
+  bool fl_list = false;        // with a tet list of its own
+  size_t o_fpo = 0, o_fch = 0, o_flist = 0;
+  DevBuf fl_corner;
   // cluster kernel: (colour, part) ranges of the elastic tets, colours with work
   size_t o_cloff = 0, o_clcol = 0, o_cllb = 0;
   int cl_nC = 0, cl_max_range = 0;
@@ -503,6 +514,23 @@ struct Solver final : SolverBase {
                    int32_t* vertex_body) override;
   int launch_groups(const LayerStatic& ls, const int* dint, const mlx_solve_params* P, int iterations,
                     const DevContacts& dc, const HostContactGroups* hc = nullptr);
+  // Dataflow path (flow.cuh): the sweeps of a layer in one launch, ordered by
+  // vertex versions.  Default where its estimate is the shortest;
+  // MLXPBD_FLOW=0 turns it off and =1 skips the estimate, and naming another
+  // launch path does too (MLXPBD_GROUPS, MLXPBD_PDL, MLXPBD_CLUSTER=1,
+  // MLXPBD_PERSISTENT=1).
+  bool flow_on = false;
+  int fl_G = 0, fl_cs = 1, fl_slots = 0, fl_smem = 0;
+  std::vector<int> fl_part;                // [T] part of each sorted tet
+  std::vector<ushort4> fl_src;             // [T] slots of its corners
+  std::vector<int> vcc_h;                  // contact_coloring: phase of each vertex's contacts
+  DevBuf fl_pin_at;
+  int plan_flow(const mlx_mesh_desc* md);
+  int flow_slots();
+  int build_flow(LayerStatic& ls, const std::vector<int>& list);
+  bool flow_layer(const LayerStatic& ls) const { return flow_on && ls.fl_ok && ls.tile.empty(); }
+  int launch_flow(const LayerStatic& ls, const int* dint, const mlx_solve_params* P, int iterations, bool pins,
+                  const DevContacts& dc, int after);
   int build_cluster_slots(LayerStatic& ls, const std::vector<int>& list);
   int launch_cluster(const LayerStatic& ls, const int* dint, const LayerDev& L, const ContactData& cd,
                      const mlx_solve_params* P, int iterations, bool body_work, LayerWork& w);
@@ -566,6 +594,10 @@ struct Solver final : SolverBase {
           if (b > 0) { lo = std::min(lo, b); hi = std::max(hi, b); }
       if (hi > 0) t = ", autotuned tiles " + std::to_string(lo) + "-" + std::to_string(hi) + " threads";
     }
+    if (flow_on && t.empty())
+      return "dataflow sweeps, one launch each: " + std::to_string(fl_G) + " clusters of " + std::to_string(fl_cs) +
+             " CTAs each owning whole components (records in shared memory); layers they do not cover: one launch per "
+             "colour (programmatic dependent launches)";
     return std::string("one launch per colour") + (pdl ? " (programmatic dependent launches)" : "") + t;
   }
   long long launches_last_call() const override { return last_launches; }
@@ -660,6 +692,10 @@ int Solver<R>::create(const mlx_mesh_desc* md) {
   for (int c = 1; c <= C; ++c) color_off[c] = color_off[c - 1] + cnt[c];
   MeshPartition mp;
   CHECK(plan_cluster(md, mp));
+  {
+    const char* e = std::getenv("MLXPBD_PERSISTENT");
+    persistent = e && std::string(e) == "1";
+  }
   // sorted order: by colour, then (cluster path) by part, then element id.
   // Tets of one colour share no vertex, so their order changes no result.
   s2e.assign(T, 0);
@@ -736,12 +772,11 @@ int Solver<R>::create(const mlx_mesh_desc* md) {
   CHECK(d_scalar.ensure(sizeof(double) * 8));  // [0] residual, [1] norm of resv, [7] k_residual_monitor's ticket
   CU(cudaMemsetAsync(d_scalar.p, 0, sizeof(double) * 8, stream));
   CHECK(h_scalar.ensure(sizeof(double) * 8));
-  CHECK(d_gsync.ensure(sizeof(unsigned int) * 4));
-  CHECK(h_gsync.ensure(sizeof(int) * 4));
-  CU(cudaMemsetAsync(d_gsync.p, 0, sizeof(unsigned int) * 4, stream));
+  // [0..3] grid barrier of the persistent kernel, [4] error flag of the dataflow path
+  CHECK(d_gsync.ensure(sizeof(unsigned int) * 8));
+  CHECK(h_gsync.ensure(sizeof(int) * 8));
+  CU(cudaMemsetAsync(d_gsync.p, 0, sizeof(unsigned int) * 8, stream));
   {
-    const char* e = std::getenv("MLXPBD_PERSISTENT");
-    persistent = e && std::string(e) == "1";
     const char* q = std::getenv("MLXPBD_PDL");
     pdl = !(q && std::string(q) == "0");
     const char* hgv = std::getenv("MLXPBD_HOST_GRAPH");
@@ -764,7 +799,8 @@ int Solver<R>::create(const mlx_mesh_desc* md) {
     CU(cudaMemcpyAsync(d_pin_dofs.p, pinned.data(), sizeof(int) * pinned.size(), cudaMemcpyHostToDevice, stream));
   vid_sorted = vid;
   if (cluster_ok) vowner = mp.vowner;
-  CHECK(plan_groups(md));
+  CHECK(plan_flow(md));
+  if (!flow_on) CHECK(plan_groups(md));
   if (md->mu && md->lambda) {
     pcg_G.resize(9 * (size_t)T);
     pcg_vol.resize(T);
@@ -1213,6 +1249,371 @@ int Solver<R>::launch_groups(const LayerStatic& ls, const int* dint, const mlx_s
   return MLX_OK;
 }
 
+// Plan of the dataflow path: how many groups of whole components, on clusters
+// of how many CTAs, and the part of every element.
+template <typename R>
+int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
+  const char* env = std::getenv("MLXPBD_FLOW");
+  const bool force = env && std::string(env) == "1";
+  if ((env && std::string(env) == "0") || persistent || cluster_ok || std::getenv("MLXPBD_PDL")) return MLX_OK;
+  if (!force && std::getenv("MLXPBD_GROUPS")) return MLX_OK;
+  // components in element order; elements of one component that are not
+  // consecutive make the whole mesh one component
+  std::vector<int> parent(N), comp_first;  // first element of every component
+  for (int v = 0; v < N; ++v) parent[v] = v;
+  auto find = [&](int v) {
+    while (parent[v] != v) {
+      parent[v] = parent[parent[v]];
+      v = parent[v];
+    }
+    return v;
+  };
+  for (int e = 0; e < T; ++e) {
+    const int a = find(md->t[e] - 1);
+    for (int k = 1; k < 4; ++k) {
+      const int b = find(md->t[e + (size_t)k * T] - 1);
+      if (a != b) parent[std::max(a, b)] = std::min(a, b);
+    }
+  }
+  {
+    std::vector<unsigned char> seen(N, 0);
+    int last = -1;
+    for (int e = 0; e < T; ++e) {
+      const int r = find(md->t[e] - 1);
+      if (r == last) continue;
+      if (seen[r]) {
+        comp_first.assign(1, 0);
+        break;
+      }
+      seen[r] = 1;
+      last = r;
+      comp_first.push_back(e);
+    }
+  }
+  const int ncomp = (int)comp_first.size();
+  comp_first.push_back(T);
+  int optin = 0;
+  CU(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+  const void* fn[2] = {flow_kernel(sizeof(R) == 8, mat_kind, damp, false), flow_kernel(sizeof(R) == 8, mat_kind, damp, true)};
+  for (const void* f : fn) {
+    cudaFuncAttributes fa;
+    CU(cudaFuncGetAttributes(&fa, f));
+    CU(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    fl_smem = optin - 1024 - (int)fa.sharedSizeBytes;  // (the kernels have no static shared memory)
+    CU(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, fl_smem));
+  }
+  int want_cs = 0;
+  if (const char* q = std::getenv("MLXPBD_FLOW_CS")) want_cs = std::atoi(q);
+  struct Plan {
+    std::vector<int> first;  // [G cs + 1] first position of every part in the element order
+    int G = 0, cs = 0, slots = 0;
+    long long sum = 0, most = 0;  // vertices summed over the parts, largest part's tets
+    double t = -1;
+  } best;
+  std::vector<int> stamp(N), order;
+  // vertices of every part of a plan
+  auto count = [&](Plan& pl) {
+    std::fill(stamp.begin(), stamp.end(), -1);
+    pl.slots = 0;
+    pl.sum = 0;
+    for (int p = 0; p < pl.G * pl.cs; ++p) {
+      int n = 0;
+      for (int i = pl.first[p]; i < pl.first[p + 1]; ++i) {
+        const int e = order.empty() ? i : order[i];
+        for (int k = 0; k < 4; ++k) {
+          int& s = stamp[md->t[e + (size_t)k * T] - 1];
+          if (s != p) {
+            s = p;
+            ++n;
+          }
+        }
+      }
+      pl.slots = std::max(pl.slots, n);
+      pl.sum += n;
+    }
+  };
+  for (int cs : {1, 2, 4, 8, 16}) {
+    if (want_cs > 0 && cs != want_cs) continue;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cs);
+    cfg.blockDim = dim3(flow_threads<R>());
+    cfg.dynamicSmemBytes = (size_t)fl_smem;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = cs;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int resident = 0;
+    if (cudaOccupancyMaxActiveClusters(&resident, fn[0], &cfg) != cudaSuccess || resident < 1) {
+      cudaGetLastError();
+      continue;
+    }
+    Plan pl;
+    pl.G = std::min(ncomp, resident);
+    pl.cs = cs;
+    for (int g = 0, c = 0; g < pl.G; ++g) {
+      // whole components up to an even share of what is left
+      const int b = comp_first[c], left = pl.G - g;
+      const long long share = (T - b + left - 1) / left;
+      int e = c + 1;
+      while (ncomp - e > left - 1 && comp_first[e] - b < share) {
+        // (the component that reaches the share stays out when that is closer)
+        if (comp_first[e + 1] - b - share > share - (comp_first[e] - b)) break;
+        ++e;
+      }
+      if (left == 1) e = ncomp;
+      const long long n = comp_first[e] - b;
+      for (int r = 0; r < cs; ++r) pl.first.push_back(b + (int)(n * r / cs));
+      pl.most = std::max(pl.most, (n + cs - 1) / cs);
+      c = e;
+    }
+    pl.first.push_back(T);
+    // Measured (B200, Neo-Hookean FP32, us per sweep): 0.9 per colour while the
+    // warps wait for records, 0.13 per chunk of the largest part while they
+    // share the SM, and both add up like independent parts (27,648 tets on
+    // 16 / 8 CTAs: 29 / 34; 10,368 on 4 / 2 / 1: 30 / 35 / 46; 98,304 on 16: 41;
+    // 393,216 on 16: 112).
+    const double chain = 0.9 * C, issue = 0.13 * ((double)pl.most / 32.0 + 0.5 * C);
+    pl.t = std::sqrt(chain * chain + issue * issue);
+    if (best.t >= 0 && pl.t >= 0.97 * best.t) continue;
+    count(pl);
+    // barriers: every colour rounds its chunks up in every part
+    const long long bars = pl.most / 32 + C;
+    if (pl.slots > kFlowMaxSlots || bars > kFlowMaxChunks || pl.slots * (long long)sizeof(R4<R>) + 8 * bars > fl_smem) continue;
+    best = pl;
+  }
+  // one launch per colour: ~1.75 us each on 98 k tets (NH FP32) plus the
+  // traffic of its tets, 85 us per sweep on 393 k
+  if (best.t < 0 || (!force && best.t > 1.75 * C + 8e-5 * (double)T)) return MLX_OK;
+  if (best.cs > 1 && best.sum > 3 * (long long)N / 2) {
+    // parts that share many vertices (an element order of thin slabs): cut
+    // the breadth-first order instead where that shares fewer
+    Plan pl = best;
+    breadth_first_elements(N, T, md->t, order);
+    bool whole = true;  // the components stay where they are in the new order
+    for (int c = 0; c < ncomp && whole; ++c)
+      for (int i = comp_first[c]; i < comp_first[c + 1] && whole; ++i)
+        whole = order[i] >= comp_first[c] && order[i] < comp_first[c + 1];
+    if (whole) count(pl);
+    if (whole && pl.sum < best.sum && pl.slots <= best.slots) best = pl;
+    else order.clear();
+  }
+  flow_on = true;
+  fl_G = best.G;
+  fl_cs = best.cs;
+  fl_slots = std::max(best.slots, 1);
+  std::vector<int> epart(T);
+  for (int p = 0; p < fl_G * fl_cs; ++p)
+    for (int i = best.first[p]; i < best.first[p + 1]; ++i) epart[order.empty() ? i : order[i]] = p;
+  fl_part.resize(T);
+  for (int s = 0; s < T; ++s) fl_part[s] = epart[s2e[s]];
+  return flow_slots();
+}
+
+// Slots of the corners of every sorted tet (each part numbers the vertices
+// its tets touch, in an order that spreads neighbours over the shared-memory
+// banks) and the pinned DOFs by vertex.
+template <typename R>
+int Solver<R>::flow_slots() {
+  std::vector<unsigned short> perm(fl_slots);
+  for (int q = 0; q < fl_slots; ++q) perm[q] = (unsigned short)q;
+  for (unsigned q = fl_slots - 1, x = 1; q > 0; --q) {
+    x = x * 1664525u + 1013904223u;
+    std::swap(perm[q], perm[(x >> 8) % (q + 1)]);
+  }
+  const int P = fl_G * fl_cs;
+  std::vector<int> off(P + 1, 0), byp(T), stamp(N, -1), slot(N);
+  for (int s = 0; s < T; ++s) ++off[fl_part[s] + 1];
+  for (int p = 0; p < P; ++p) off[p + 1] += off[p];
+  {
+    std::vector<int> f(off.begin(), off.end() - 1);
+    for (int s = 0; s < T; ++s) byp[f[fl_part[s]]++] = s;
+  }
+  fl_src.assign(T, make_ushort4(0, 0, 0, 0));
+  for (int p = 0; p < P; ++p) {
+    int n = 0;
+    for (int i = off[p]; i < off[p + 1]; ++i) {
+      const int s = byp[i];
+      const int4 v4 = vid_sorted[s];
+      const int v[4] = {v4.x, v4.y, v4.z, v4.w};
+      unsigned short q[4];
+      for (int k = 0; k < 4; ++k) {
+        if (stamp[v[k]] != p) {
+          stamp[v[k]] = p;
+          slot[v[k]] = n++;
+        }
+        q[k] = perm[slot[v[k]]];
+      }
+      fl_src[s] = make_ushort4(q[0], q[1], q[2], q[3]);
+    }
+  }
+  if (!pinned.empty()) {
+    std::vector<int> at(3 * (size_t)N, -1);
+    for (size_t i = 0; i < pinned.size(); ++i) at[pinned[i]] = (int)i;
+    CHECK(fl_pin_at.ensure(sizeof(int) * at.size()));
+    CU(cudaMemcpyAsync(fl_pin_at.p, at.data(), sizeof(int) * at.size(), cudaMemcpyHostToDevice, stream));
+    CU(cudaStreamSynchronize(stream));
+  }
+  return MLX_OK;
+}
+
+// Chunks, corner words and slots of one layer's elastic tets (`list`: their
+// sorted ids in colour order).
+template <typename R>
+int Solver<R>::build_flow(LayerStatic& ls, const std::vector<int>& clist) {
+  const int P = fl_G * fl_cs;
+  // the layer's list in (colour, part) order; the sorted order already is
+  // that when the parts are runs of the element order
+  std::vector<int> list = clist;
+  ls.fl_list = false;
+  {
+    std::vector<int> at(P + 1);
+    for (int c = 0; c < C; ++c) {
+      const int b = ls.color_start[c], n = ls.color_count[c];
+      std::fill(at.begin(), at.end(), 0);
+      bool run = true;
+      for (int o = 0; o < n; ++o) {
+        ++at[fl_part[clist[b + o]] + 1];
+        run = run && (o == 0 || fl_part[clist[b + o]] >= fl_part[clist[b + o - 1]]);
+      }
+      if (run) continue;
+      ls.fl_list = true;
+      for (int p = 0; p < P; ++p) at[p + 1] += at[p];
+      for (int o = 0; o < n; ++o) list[b + at[fl_part[clist[b + o]]]++] = clist[b + o];
+    }
+  }
+  std::vector<FlowCorner> corner(T);
+  std::vector<int> last(N, -1);      // corner (4 s + k) of the vertex's latest tet
+  std::vector<unsigned> home(N, 0);  // where its first tet reads it
+  std::vector<unsigned char> pin(N, 0), taken(N, 0);
+  for (int d : pinned) pin[d / 3] = 1;
+  ls.fl_coloured = !vcc_h.empty();
+  std::vector<std::vector<int4>> chunks(P);
+  std::vector<int> first_chunk(N, -1), first_part(N, -1), last_part(N, -1);  // of the vertex's first / latest tet
+  for (int c = 0; c < C; ++c) {
+    const int b = ls.color_start[c], n = ls.color_count[c];
+    const int at = ls.identity_list && !ls.fl_list ? color_off[c] : b;
+    for (int o = 0; o < n;) {
+      const int p = fl_part[list[b + o]], j = (int)chunks[p].size();
+      const unsigned me = (unsigned)(p % fl_cs) << 28 | (unsigned)j << 14;
+      int4 ch = make_int4(at + o, 0, 0, 0);
+      for (; ch.y < 32 && o + ch.y < n && fl_part[list[b + o + ch.y]] == p; ++ch.y) {
+        const int s = list[b + o + ch.y];
+        const int4 v4 = vid_sorted[s];
+        const ushort4 q4 = fl_src[s];
+        const int v[4] = {v4.x, v4.y, v4.z, v4.w};
+        const unsigned q[4] = {q4.x, q4.y, q4.z, q4.w};
+        for (int k = 0; k < 4; ++k) {
+          unsigned word = pin[v[k]] ? kFlowPinned : 0;
+          if (ls.rid[v[k]] == 0) word |= kFlowFree;
+          if (ls.fl_coloured && ls.rid[v[k]] == 0 && !taken[v[k]] && c > vcc_h[v[k]]) {
+            taken[v[k]] = 1;
+            word |= kFlowBefore;
+          }
+          const int l = last[v[k]];
+          if (l >= 0) {
+            corner[l >> 2].c[l & 3].y = me | q[k];
+            if (last_part[v[k]] == p) ++ch.w;
+            else ++ch.z;
+          } else {
+            home[v[k]] = me | q[k];
+            first_chunk[v[k]] = j;
+            first_part[v[k]] = p;
+            word |= kFlowFirst;
+          }
+          last[v[k]] = 4 * s + k;
+          last_part[v[k]] = p;
+          corner[s].c[k] = make_uint2(q[k] | word << 16, 0);
+        }
+      }
+      chunks[p].push_back(ch);
+      o += ch.y;
+    }
+  }
+  ls.fl_loose_pins = ls.fl_loose_free = false;
+  for (int v = 0; v < N; ++v) {
+    if (last[v] < 0) {
+      if (pin[v]) ls.fl_loose_pins = true;
+      if (ls.rid[v] == 0) ls.fl_loose_free = true;
+      continue;
+    }
+    uint2& w = corner[last[v] >> 2].c[last[v] & 3];
+    w.y = home[v];
+    // the first tet's record comes from the last one, from iteration 1 on
+    if (last_part[v] == first_part[v]) chunks[first_part[v]][first_chunk[v]].w += 1 | 1 << 16;
+    w.x |= kFlowLast << 16;
+    // coloured contacts after every tet of this layer; phase C (no free
+    // colour) is the body phase's when the layer has bodies
+    if (ls.fl_coloured && ls.rid[v] == 0 && !taken[v] && (vcc_h[v] < C || ls.nb == 0)) w.x |= kFlowAfter << 16;
+  }
+  std::vector<int> off(P + 1, 0), flat;
+  for (int p = 0; p < P; ++p) {
+    off[p + 1] = off[p] + (int)chunks[p].size();
+    for (const int4& ch : chunks[p]) flat.insert(flat.end(), {ch.x, ch.y, ch.z, ch.w});
+  }
+  ls.fl_chunks = off[P];
+  ls.fl_max = 0;
+  for (int p = 0; p < P; ++p) ls.fl_max = std::max(ls.fl_max, off[p + 1] - off[p]);
+  if ((size_t)fl_slots * sizeof(R4<R>) + 8 * (size_t)ls.fl_max > (size_t)fl_smem || ls.fl_max > kFlowMaxChunks)
+    return MLX_OK;
+  ls.o_flist = ls.packed.size();
+  if (ls.fl_list) ls.packed.insert(ls.packed.end(), list.begin(), list.end());
+  ls.o_fpo = ls.packed.size();
+  ls.packed.insert(ls.packed.end(), off.begin(), off.end());
+  while (ls.packed.size() & 3) ls.packed.push_back(0);  // int4 alignment
+  ls.o_fch = ls.packed.size();
+  ls.packed.insert(ls.packed.end(), flat.begin(), flat.end());
+  CHECK(ls.fl_corner.ensure(sizeof(FlowCorner) * (size_t)T));
+  CU(cudaMemcpyAsync(ls.fl_corner.p, corner.data(), sizeof(FlowCorner) * (size_t)T, cudaMemcpyHostToDevice, stream));
+  CU(cudaStreamSynchronize(stream));
+  ls.fl_ok = true;
+  return MLX_OK;
+}
+
+template <typename R>
+int Solver<R>::launch_flow(const LayerStatic& ls, const int* dint, const mlx_solve_params* P, int iterations, bool pins,
+                           const DevContacts& dc, int after) {
+  if (ls.fl_chunks == 0) return MLX_OK;
+  FlowArgs<R> a;
+  a.part_off = dint + ls.o_fpo;
+  a.chunks = reinterpret_cast<const int4*>(dint + ls.o_fch);
+  a.list = ls.fl_list ? dint + ls.o_flist : (ls.identity_list ? nullptr : dint + ls.o_list);
+  a.corner = ls.fl_corner.template as<FlowCorner>();
+  a.pin_at = fl_pin_at.as<int>();
+  a.pin_vals = d_pinx.as<R>();
+  a.error = reinterpret_cast<int*>(d_gsync.as<unsigned int>() + 4);
+  a.cs = fl_cs;
+  a.slots = fl_slots;
+  a.iterations = iterations;
+  a.pins = pins && !pinned.empty() ? 1 : 0;
+  a.after = after;
+  a.h = P->h;
+  a.contact_resistance = P->contact_resistance;
+  TetData<R> td = tets();
+  R4<R>* p = pos();
+  const R4<R>* oldp = d_oldp.as<R4<R>>();
+  const R h = (R)P->h;
+  R inv_h2 = R(1) / (h * h), inv_h = R(1) / h;
+  DevContacts dcv = dc;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(fl_G * fl_cs);
+  cfg.blockDim = dim3(32 * std::min(flow_threads<R>() / 32, ls.fl_max));
+  cfg.dynamicSmemBytes = (size_t)fl_slots * sizeof(R4<R>) + 8 * (size_t)ls.fl_max;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = fl_cs;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  void* args[] = {&td, &a, &p, &oldp, &inv_h2, &inv_h, &dcv};
+  const cudaError_t e =
+      cudaLaunchKernelExC(&cfg, after ? flow_kernel(sizeof(R) == 8, mat_kind, damp, true) : flow_kernel(sizeof(R) == 8, mat_kind, damp, false), args);
+  if (e != cudaSuccess) return set_error(MLX_ERR_CUDA, std::string("dataflow sweep launch: ") + cudaGetErrorString(e));
+  return MLX_OK;
+}
+
 // Diagnostic of the grid barrier's bounded wait: thread 0 waits for a count
 // nothing increments, so the wait runs out after limit_ns.
 __global__ void k_probe_grid_wait(unsigned* count, int* error, unsigned long long limit_ns, int* timed_out) {
@@ -1508,6 +1909,8 @@ int Solver<R>::build_static(const mlx_layer_desc* ld, int col, LayerStatic& ls, 
       ls.gr_ok = true;
     }
   }
+  ls.fl_ok = false;
+  if (flow_on) CHECK(build_flow(ls, list));
   if (cluster_ok) {
     // the elastic list (or the identity) is in sorted order, which is
     // (colour, part) order on the cluster path
@@ -2032,6 +2435,36 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
       }
       continue;
     }
+    // the sweep as one launch (flow.cuh): without bodies it also takes the
+    // device-detected contacts and the pins, and a fixed number of iterations
+    const bool flowDev = dc.nobs > 0 && (ls.nb == 0 || dc.colored);  // contacts inside the sweep
+    const bool flow = flow_layer(ls) && (!flowDev || (!ls.fl_loose_free && (!dc.colored || ls.fl_coloured)));
+    const int flowAfter = !flowDev ? 0 : (dc.colored ? 2 : 1);
+    const bool flowAll = flow && ls.nb == 0 && nK == 0;  // nothing but the sweep, its contacts and the pins
+    if (flowAll && !P->compute_residuals) {
+      const int iters = std::max(ld->iterations[layer], 0);
+      if (iters > 0) {
+        const bool timed = sweep_timing && tev_used + 2 <= tev.size();
+        if (timed) CHECK(record_event(tev[tev_used], capturing));
+        CHECK(launch_flow(ls, dint, P, iters, true, dc, flowAfter));
+        if (timed) {
+          double b = 0;
+          for (int c = 0; c < C; ++c) b += ls.color_count[c] * (group_bytes_per_tet() + (ls.identity_list ? 0.0 : 4.0));
+          CHECK(record_event(tev[tev_used + 1], capturing));
+          tev_bytes[tev_used / 2] = b * iters + 2.0 * (double)N * sizeof(R4<R>);
+          tev_launches[tev_used / 2] = 1;
+          tev_used += 2;
+        }
+        ++st.launches;
+        st.totalIterations += iters;
+        if (np && ls.fl_loose_pins) {
+          k_pin<R><<<blocks_for((long long)np, 256), 256, 0, stream>>>(p, d_pin_dofs.as<int>(), d_pinx.as<R>(), (int)np);
+          CU(cudaGetLastError());
+          ++st.launches;
+        }
+      }
+      continue;
+    }
     cudaGraphConditionalHandle h_while_cur = 0;
     if (devmon) {
       // the projectGS loop as a WHILE node whose body is one iteration
@@ -2054,7 +2487,13 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
       if (timed) CHECK(record_event(tev[tev_used], capturing));
       long long sweep_l = 0;
       double sweep_b = 0;
-      for (int c = 0; c < C; ++c) {
+      if (flow) {
+        CHECK(launch_flow(ls, dint, P, 1, flowAll, dc, flowAfter));
+        ++st.launches;
+        sweep_l = 1;
+        for (int c = 0; c < C; ++c) sweep_b += ls.color_count[c] * (bytes_per_tet() + (ls.identity_list ? 0.0 : 4.0));
+      }
+      for (int c = 0; c < C && !flow; ++c) {
         if (ls.color_count[c] == 0 && !dc.colored) continue;
         CHECK(launch_color(c, ls, dlist, hR, 0, dc.colored ? &dc : nullptr, L.vert_body, h, P->contact_resistance));
         ++st.launches;
@@ -2067,7 +2506,7 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
         tev_launches[tev_used / 2] = sweep_l;
         tev_used += 2;
       }
-      if (bodyWork) {
+      if (bodyWork && !flowAll) {
         cudaLaunchConfig_t cfg = pdl_config((ls.nb > 0 ? ls.n_items : 0) + ecBlocks, kBodyThreads);
         cudaLaunchAttribute attr = pdl_attr();
         cfg.attrs = &attr;
@@ -2078,7 +2517,7 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
                               (const R4<R>*)d_oldp.as<R4<R>>()));
         ++st.launches;
       }
-      if (np) {
+      if (np && (!flowAll || ls.fl_loose_pins)) {
         cudaLaunchConfig_t cfg = pdl_config(blocks_for((long long)np, 256), 256);
         cudaLaunchAttribute attr = pdl_attr();
         cfg.attrs = &attr;
@@ -2283,6 +2722,11 @@ template <typename R>
 int Solver<R>::check_gsync() {
   if (h_gsync.as<int>()[2] != 0)
     return set_error(MLX_ERR_LIMIT, "a grid barrier of the persistent layer kernel waited more than 1 s");
+  if (h_gsync.as<int>()[4] != 0) {
+    // (kept across the steps of a call; cleared once reported)
+    CU(cudaMemsetAsync(d_gsync.as<unsigned int>() + 4, 0, sizeof(int), stream));
+    return set_error(MLX_ERR_LIMIT, "a tet of a sweep waited more than 1 s for a vertex");
+  }
   return MLX_OK;
 }
 
@@ -2660,7 +3104,7 @@ int Solver<R>::layer_solve(const mlx_layer_desc* ld, const mlx_solve_params* P, 
     hg.lkey = lkey;
     hg.pkey = pkey;
   }
-  CU(cudaMemcpyAsync(h_gsync.p, d_gsync.p, sizeof(unsigned int) * 4, cudaMemcpyDeviceToHost, stream));
+  CU(cudaMemcpyAsync(h_gsync.p, d_gsync.p, sizeof(unsigned int) * 8, cudaMemcpyDeviceToHost, stream));
   // ---- download ----
   k_store_pos<R><<<blocks_for(N, bs), bs, 0, stream>>>(pos(), ds, N);
   if (out->lambdai) k_store_lambda<R><<<blocks_for(T, bs), bs, 0, stream>>>(d_lambda.as<R>(), d_s2e.as<int>(), ds + n3, T);
@@ -2772,6 +3216,7 @@ int Solver<R>::sim_setup(const mlx_layer_desc* ld, const mlx_solve_params* P, co
   sim.ld.is_rigid_vertex = sim.isRV.data();
   sim.ld.num_rigids = sim.nr.data();
   sim.P = *P;
+  if (P->contact_coloring) CHECK(contact_colours());
   // build every column once and reserve the body buffers for capture
   if (sim.graph) { cudaGraphExecDestroy(sim.graph); sim.graph = nullptr; }
   sim_work.cache.clear();
@@ -2997,6 +3442,7 @@ int Solver<R>::contact_colours() {
         vcc[v] = c;
         break;
       }
+  vcc_h = vcc;
   CHECK(d_vcc.ensure(sizeof(int) * (size_t)N));
   CHECK(d_cbucket.ensure(sizeof(int) * (size_t)N));
   CHECK(d_coff.ensure(sizeof(int) * (size_t)(C + 2)));
@@ -3748,7 +4194,7 @@ int Solver<R>::sim_issue_step(long long* launches, bool capturing) {
     CU(cudaGetLastError());
     ++st.launches;
   }
-  CU(cudaMemcpyAsync(h_gsync.p, d_gsync.p, sizeof(unsigned int) * 4, cudaMemcpyDeviceToHost, stream));
+  CU(cudaMemcpyAsync(h_gsync.p, d_gsync.p, sizeof(unsigned int) * 8, cudaMemcpyDeviceToHost, stream));
   if (launches) *launches = st.launches + 2;
   return MLX_OK;
 }
