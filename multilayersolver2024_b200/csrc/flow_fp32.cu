@@ -1,8 +1,10 @@
-// flow_fp32.cu -- k_flow with FP32 storage.
+// flow_fp32.cu -- the one-launch sweeps with FP32 storage.
 #include "flow_kernel.cuh"
+#include "sweep_kernel.cuh"
 
 namespace mlx {
 const void* flow_kernel_fp32(int mat_kind, bool damp, bool ct) {
   return ct ? flow_kernel_of<float, true>(mat_kind, damp) : flow_kernel_of<float, false>(mat_kind, damp);
 }
+const void* sweep_kernel_fp32(int mat_kind, bool damp) { return sweep_kernel_of<float>(mat_kind, damp); }
 }  // namespace mlx

@@ -1,8 +1,10 @@
-// flow_fp64.cu -- k_flow with FP64 storage.
+// flow_fp64.cu -- the one-launch sweeps with FP64 storage.
 #include "flow_kernel.cuh"
+#include "sweep_kernel.cuh"
 
 namespace mlx {
 const void* flow_kernel_fp64(int mat_kind, bool damp, bool ct) {
   return ct ? flow_kernel_of<double, true>(mat_kind, damp) : flow_kernel_of<double, false>(mat_kind, damp);
 }
+const void* sweep_kernel_fp64(int mat_kind, bool damp) { return sweep_kernel_of<double>(mat_kind, damp); }
 }  // namespace mlx

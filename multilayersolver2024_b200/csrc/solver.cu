@@ -18,6 +18,7 @@
 #include "cluster.cuh"
 #include "groups.cuh"
 #include "flow.cuh"
+#include "sweep.cuh"
 #include "layers_dev.cuh"
 #include "contacts.cuh"
 #include "monitor.cuh"
@@ -220,12 +221,17 @@ struct LayerStatic {
   // dataflow path (flow.cuh): chunks of each part, corner words and slots
   bool fl_ok = false;
   int fl_chunks = 0, fl_max = 0;  // chunks, largest part's
-  bool fl_loose_pins = false;  // a pinned vertex has no elastic tet in this layer
+  bool loose_pins = false;     // a pinned vertex has no elastic tet in this layer
   bool fl_loose_free = false;  // a vertex of no body has none
   bool fl_coloured = false;    // the corner words hold the contact phases
   bool fl_list = false;        // with a tet list of its own
   size_t o_fpo = 0, o_fch = 0, o_flist = 0;
   DevBuf fl_corner;
+  // sweeps through L2 (sweep.cuh): chunks and corner words
+  bool sw_ok = false;
+  int sw_chunks = 0, sw_D = 0;
+  size_t o_swch = 0;
+  DevBuf sw_corner;
   // cluster kernel: (colour, part) ranges of the elastic tets, colours with work
   size_t o_cloff = 0, o_clcol = 0, o_cllb = 0;
   int cl_nC = 0, cl_max_range = 0;
@@ -527,10 +533,24 @@ struct Solver final : SolverBase {
   DevBuf fl_pin_at;
   int plan_flow(const mlx_mesh_desc* md);
   int flow_slots();
+  int upload_pin_at();
   int build_flow(LayerStatic& ls, const std::vector<int>& list);
   bool flow_layer(const LayerStatic& ls) const { return flow_on && ls.fl_ok && ls.tile.empty(); }
   int launch_flow(const LayerStatic& ls, const int* dint, const mlx_solve_params* P, int iterations, bool pins,
                   const DevContacts& dc, int after);
+  // The sweeps of a layer in one launch over the whole GPU, versions through
+  // L2 (sweep.cuh): components too large for the dataflow path's clusters.
+  // MLXPBD_FLOW=0 and the other switches above turn it off too,
+  // MLXPBD_FLOW=2 skips the estimate.
+  bool sweep_on = false;
+  int sw_sms = 0;
+  DevBuf sw_rec, sw_minv, sw_state;
+  int plan_sweep();
+  int build_sweep(LayerStatic& ls, const std::vector<int>& list);
+  bool sweep_layer(const LayerStatic& ls, int iterations) const {
+    return sweep_on && ls.sw_ok && ls.tile.empty() && (long long)ls.sw_D * std::max(iterations, 1) < kSweepMaxTags;
+  }
+  int launch_sweep(const LayerStatic& ls, const int* dint, R h, int iterations, bool pins);
   int build_cluster_slots(LayerStatic& ls, const std::vector<int>& list);
   int launch_cluster(const LayerStatic& ls, const int* dint, const LayerDev& L, const ContactData& cd,
                      const mlx_solve_params* P, int iterations, bool body_work, LayerWork& w);
@@ -594,6 +614,9 @@ struct Solver final : SolverBase {
           if (b > 0) { lo = std::min(lo, b); hi = std::max(hi, b); }
       if (hi > 0) t = ", autotuned tiles " + std::to_string(lo) + "-" + std::to_string(hi) + " threads";
     }
+    if (sweep_on && t.empty())
+      return "version-ordered sweeps, one launch each on " + std::to_string(sw_sms) +
+             " CTAs; contacts coloured with the elastic constraints: one launch per colour";
     if (flow_on && t.empty())
       return "dataflow sweeps, one launch each: " + std::to_string(fl_G) + " clusters of " + std::to_string(fl_cs) +
              " CTAs each owning whole components (records in shared memory); layers they do not cover: one launch per "
@@ -800,7 +823,7 @@ int Solver<R>::create(const mlx_mesh_desc* md) {
   vid_sorted = vid;
   if (cluster_ok) vowner = mp.vowner;
   CHECK(plan_flow(md));
-  if (!flow_on) CHECK(plan_groups(md));
+  if (!flow_on && !sweep_on) CHECK(plan_groups(md));
   if (md->mu && md->lambda) {
     pcg_G.resize(9 * (size_t)T);
     pcg_vol.resize(T);
@@ -1256,6 +1279,7 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
   const char* env = std::getenv("MLXPBD_FLOW");
   const bool force = env && std::string(env) == "1";
   if ((env && std::string(env) == "0") || persistent || cluster_ok || std::getenv("MLXPBD_PDL")) return MLX_OK;
+  if (env && std::string(env) == "2") return plan_sweep();
   if (!force && std::getenv("MLXPBD_GROUPS")) return MLX_OK;
   // components in element order; elements of one component that are not
   // consecutive make the whole mesh one component
@@ -1383,9 +1407,11 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
     if (pl.slots > kFlowMaxSlots || bars > kFlowMaxChunks || pl.slots * (long long)sizeof(R4<R>) + 8 * bars > fl_smem) continue;
     best = pl;
   }
-  // one launch per colour: ~1.75 us each on 98 k tets (NH FP32) plus the
-  // traffic of its tets, 85 us per sweep on 393 k
-  if (best.t < 0 || (!force && best.t > 1.75 * C + 8e-5 * (double)T)) return MLX_OK;
+  // A launch per colour takes ~1.75 us plus its tets' traffic (58 us per sweep
+  // of 98 k tets, 85 of 393 k), the sweep through L2 less than that at any
+  // size (53 and 62 us).
+  if (!force && (best.t < 0 || best.t > 1.55 * C + 3.3e-5 * (double)T)) return plan_sweep();
+  if (best.t < 0) return MLX_OK;
   if (best.cs > 1 && best.sum > 3 * (long long)N / 2) {
     // parts that share many vertices (an element order of thin slabs): cut
     // the breadth-first order instead where that shares fewer
@@ -1448,13 +1474,131 @@ int Solver<R>::flow_slots() {
       fl_src[s] = make_ushort4(q[0], q[1], q[2], q[3]);
     }
   }
-  if (!pinned.empty()) {
-    std::vector<int> at(3 * (size_t)N, -1);
-    for (size_t i = 0; i < pinned.size(); ++i) at[pinned[i]] = (int)i;
-    CHECK(fl_pin_at.ensure(sizeof(int) * at.size()));
-    CU(cudaMemcpyAsync(fl_pin_at.p, at.data(), sizeof(int) * at.size(), cudaMemcpyHostToDevice, stream));
-    CU(cudaStreamSynchronize(stream));
+  return upload_pin_at();
+}
+
+template <typename R>
+int Solver<R>::upload_pin_at() {
+  if (pinned.empty()) return MLX_OK;
+  std::vector<int> at(3 * (size_t)N, -1);
+  for (size_t i = 0; i < pinned.size(); ++i) at[pinned[i]] = (int)i;
+  CHECK(fl_pin_at.ensure(sizeof(int) * at.size()));
+  CU(cudaMemcpyAsync(fl_pin_at.p, at.data(), sizeof(int) * at.size(), cudaMemcpyHostToDevice, stream));
+  CU(cudaStreamSynchronize(stream));
+  return MLX_OK;
+}
+
+// Buffers of the sweep through L2: the corners' inverse masses, the vertex
+// records and their tag counter.
+template <typename R>
+int Solver<R>::plan_sweep() {
+  if (C > kSweepRank) return MLX_OK;
+  int per_sm = 0;
+  CU(cudaDeviceGetAttribute(&sw_sms, cudaDevAttrMultiProcessorCount, device));
+  CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sweep_kernel(sizeof(R) == 8, mat_kind, damp), kSweepThreads, 0));
+  if (per_sm < 1) return MLX_OK;
+  CHECK(sw_rec.ensure(sizeof(SweepRec<R>) * (size_t)N));
+  CHECK(sw_state.ensure(sizeof(SweepState)));
+  CU(cudaMemsetAsync(sw_rec.p, 0, sizeof(SweepRec<R>) * (size_t)N, stream));
+  CU(cudaMemsetAsync(sw_state.p, 0, sizeof(SweepState), stream));
+  std::vector<R4<R>> m4(T);
+  std::vector<R> mi(N);
+  for (int v = 0; v < N; ++v) mi[v] = (R)(1.0 / vmass_h[v]);
+  for (int s = 0; s < T; ++s) {
+    const int4 v = vid_sorted[s];
+    m4[s] = make_r4<R>(mi[v.x], mi[v.y], mi[v.z], mi[v.w]);
   }
+  CHECK(sw_minv.ensure(sizeof(R4<R>) * (size_t)T));
+  CU(cudaMemcpyAsync(sw_minv.p, m4.data(), sizeof(R4<R>) * (size_t)T, cudaMemcpyHostToDevice, stream));
+  CU(cudaStreamSynchronize(stream));
+  sweep_on = true;
+  return upload_pin_at();
+}
+
+// Chunks and corner words of one layer's elastic tets (`list`: their sorted
+// ids in colour order) for the sweep through L2.
+template <typename R>
+int Solver<R>::build_sweep(LayerStatic& ls, const std::vector<int>& list) {
+  std::vector<unsigned short> rank(N, 0);
+  std::vector<ushort4> corner(T, make_ushort4(0, 0, 0, 0));
+  for (int s : list) {
+    const int4 v = vid_sorted[s];
+    // (a colour has at most one tet of a vertex, so rank < C)
+    corner[s] = make_ushort4(rank[v.x]++, rank[v.y]++, rank[v.z]++, rank[v.w]++);
+  }
+  std::vector<unsigned char> pin(N, 0);
+  ls.loose_pins = false;
+  for (int d : pinned) {
+    pin[d / 3] = 1;
+    if (rank[d / 3] == 0) ls.loose_pins = true;
+  }
+  ls.sw_D = 1;
+  for (int v = 0; v < N; ++v) ls.sw_D = std::max(ls.sw_D, (int)rank[v]);
+  auto mark = [&](unsigned short& wd, int v) {
+    if (wd + 1 == rank[v]) wd |= kSweepLast;
+    if (pin[v]) wd |= kSweepPinned;
+  };
+  for (int s : list) {
+    const int4 v = vid_sorted[s];
+    ushort4& cw = corner[s];
+    mark(cw.x, v.x); mark(cw.y, v.y); mark(cw.z, v.z); mark(cw.w, v.w);
+  }
+  while (ls.packed.size() & 1) ls.packed.push_back(0);  // int2 alignment
+  ls.o_swch = ls.packed.size();
+  for (int c = 0; c < C; ++c) {
+    const int b = ls.identity_list ? color_off[c] : ls.color_start[c];
+    for (int o = 0; o < ls.color_count[c]; o += 32) {
+      ls.packed.push_back(b + o);
+      ls.packed.push_back(std::min(32, ls.color_count[c] - o));
+    }
+  }
+  ls.sw_chunks = (int)(ls.packed.size() - ls.o_swch) / 2;
+  CHECK(ls.sw_corner.ensure(sizeof(ushort4) * (size_t)T));
+  CU(cudaMemcpyAsync(ls.sw_corner.p, corner.data(), sizeof(ushort4) * (size_t)T, cudaMemcpyHostToDevice, stream));
+  CU(cudaStreamSynchronize(stream));
+  ls.sw_ok = true;
+  return MLX_OK;
+}
+
+template <typename R>
+int Solver<R>::launch_sweep(const LayerStatic& ls, const int* dint, R h, int iterations, bool pins) {
+  if (ls.sw_chunks == 0) return MLX_OK;
+  SweepArgs<R> a;
+  a.chunks = reinterpret_cast<const int2*>(dint + ls.o_swch);
+  a.list = ls.identity_list ? nullptr : dint + ls.o_list;
+  a.corner = ls.sw_corner.template as<ushort4>();
+  a.minv = sw_minv.as<R4<R>>();
+  a.rec = sw_rec.as<SweepRec<R>>();
+  a.state = sw_state.as<SweepState>();
+  a.error = reinterpret_cast<int*>(d_gsync.as<unsigned int>() + 4);
+  a.pin_at = fl_pin_at.as<int>();
+  a.pin_vals = d_pinx.as<R>();
+  a.n_chunks = ls.sw_chunks;
+  a.iterations = iterations;
+  a.D = ls.sw_D;
+  a.N = N;
+  a.pins = pins && !pinned.empty() ? 1 : 0;
+  // a colour's chunks per CTA: one waiting chunk at a time while a CTA has
+  // few (98 k tets: 55 us per sweep with one, 59 with two), two above that
+  // (393 k: 65 and 63); 866 k tets want eight warps (75 us; 106 with four)
+  const double per = (double)ls.sw_chunks / ((double)C * sw_sms);
+  a.gate = per < 2 ? 1 : 2;
+  TetData<R> td = tets();
+  R4<R>* p = pos();
+  const R4<R>* oldp = d_oldp.as<R4<R>>();
+  R inv_h2 = R(1) / (h * h), inv_h = R(1) / h;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(std::min(sw_sms, ls.sw_chunks));
+  cfg.blockDim = dim3(per < 4 ? kSweepThreads / 2 : kSweepThreads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  void* args[] = {&td, &a, &p, &oldp, &inv_h2, &inv_h};
+  const cudaError_t e = cudaLaunchKernelExC(&cfg, sweep_kernel(sizeof(R) == 8, mat_kind, damp), args);
+  if (e != cudaSuccess) return set_error(MLX_ERR_CUDA, std::string("sweep launch: ") + cudaGetErrorString(e));
   return MLX_OK;
 }
 
@@ -1531,10 +1675,10 @@ int Solver<R>::build_flow(LayerStatic& ls, const std::vector<int>& clist) {
       o += ch.y;
     }
   }
-  ls.fl_loose_pins = ls.fl_loose_free = false;
+  ls.loose_pins = ls.fl_loose_free = false;
   for (int v = 0; v < N; ++v) {
     if (last[v] < 0) {
-      if (pin[v]) ls.fl_loose_pins = true;
+      if (pin[v]) ls.loose_pins = true;
       if (ls.rid[v] == 0) ls.fl_loose_free = true;
       continue;
     }
@@ -1911,6 +2055,8 @@ int Solver<R>::build_static(const mlx_layer_desc* ld, int col, LayerStatic& ls, 
   }
   ls.fl_ok = false;
   if (flow_on) CHECK(build_flow(ls, list));
+  ls.sw_ok = false;
+  if (sweep_on) CHECK(build_sweep(ls, list));
   if (cluster_ok) {
     // the elastic list (or the identity) is in sorted order, which is
     // (colour, part) order on the cluster path
@@ -2440,13 +2586,15 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
     const bool flowDev = dc.nobs > 0 && (ls.nb == 0 || dc.colored);  // contacts inside the sweep
     const bool flow = flow_layer(ls) && (!flowDev || (!ls.fl_loose_free && (!dc.colored || ls.fl_coloured)));
     const int flowAfter = !flowDev ? 0 : (dc.colored ? 2 : 1);
-    const bool flowAll = flow && ls.nb == 0 && nK == 0;  // nothing but the sweep, its contacts and the pins
+    const int iters = std::max(ld->iterations[layer], 0);
+    const bool sweep = !dc.colored && sweep_layer(ls, P->compute_residuals ? 1 : iters);
+    // nothing but the sweep, its contacts and the pins
+    const bool flowAll = ls.nb == 0 && nK == 0 && (flow || (sweep && !dc.nobs));
     if (flowAll && !P->compute_residuals) {
-      const int iters = std::max(ld->iterations[layer], 0);
       if (iters > 0) {
         const bool timed = sweep_timing && tev_used + 2 <= tev.size();
         if (timed) CHECK(record_event(tev[tev_used], capturing));
-        CHECK(launch_flow(ls, dint, P, iters, true, dc, flowAfter));
+        CHECK(flow ? launch_flow(ls, dint, P, iters, true, dc, flowAfter) : launch_sweep(ls, dint, hR, iters, true));
         if (timed) {
           double b = 0;
           for (int c = 0; c < C; ++c) b += ls.color_count[c] * (group_bytes_per_tet() + (ls.identity_list ? 0.0 : 4.0));
@@ -2457,7 +2605,7 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
         }
         ++st.launches;
         st.totalIterations += iters;
-        if (np && ls.fl_loose_pins) {
+        if (np && ls.loose_pins) {
           k_pin<R><<<blocks_for((long long)np, 256), 256, 0, stream>>>(p, d_pin_dofs.as<int>(), d_pinx.as<R>(), (int)np);
           CU(cudaGetLastError());
           ++st.launches;
@@ -2487,13 +2635,13 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
       if (timed) CHECK(record_event(tev[tev_used], capturing));
       long long sweep_l = 0;
       double sweep_b = 0;
-      if (flow) {
-        CHECK(launch_flow(ls, dint, P, 1, flowAll, dc, flowAfter));
+      if (flow || sweep) {
+        CHECK(flow ? launch_flow(ls, dint, P, 1, flowAll, dc, flowAfter) : launch_sweep(ls, dint, hR, 1, flowAll));
         ++st.launches;
         sweep_l = 1;
         for (int c = 0; c < C; ++c) sweep_b += ls.color_count[c] * (bytes_per_tet() + (ls.identity_list ? 0.0 : 4.0));
       }
-      for (int c = 0; c < C && !flow; ++c) {
+      for (int c = 0; c < C && !flow && !sweep; ++c) {
         if (ls.color_count[c] == 0 && !dc.colored) continue;
         CHECK(launch_color(c, ls, dlist, hR, 0, dc.colored ? &dc : nullptr, L.vert_body, h, P->contact_resistance));
         ++st.launches;
@@ -2517,7 +2665,7 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
                               (const R4<R>*)d_oldp.as<R4<R>>()));
         ++st.launches;
       }
-      if (np && (!flowAll || ls.fl_loose_pins)) {
+      if (np && (!flowAll || ls.loose_pins)) {
         cudaLaunchConfig_t cfg = pdl_config(blocks_for((long long)np, 256), 256);
         cudaLaunchAttribute attr = pdl_attr();
         cfg.attrs = &attr;

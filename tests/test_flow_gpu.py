@@ -1,5 +1,6 @@
-"""The dataflow sweeps (flow.cuh: colours ordered by the vertices' chains,
-records pushed through shared memory) against one launch per colour: the same
+"""The one-launch sweeps (flow.cuh: colours ordered by the vertices' chains,
+records pushed through shared memory; sweep.cuh: versions through L2) against
+one launch per colour: the same
 arithmetic in the same order at every vertex, so FP32 results are equal bit
 for bit (FP64 to the compiler's choice of fused multiply-adds), and against
 the oracle.  Sizes: less than one chunk of 32 tets, ragged chunks, several
@@ -17,11 +18,12 @@ pytestmark = pytest.mark.gpu
 NH, STVK = _lib.MLX_ENERGY_NEOHOOKEAN, _lib.MLX_ENERGY_STVK_VOIGT
 
 
-def _paths(monkeypatch, make, cs=""):
-    """make() on the colour launches and on the dataflow path."""
+def _paths(monkeypatch, make, cs="", path="1"):
+    """make() on the colour launches and on the dataflow path (or, "2", the
+    sweep whose versions go through L2)."""
     out = []
     monkeypatch.setenv("MLXPBD_GROUPS", "0")
-    for flag in ("0", "1"):
+    for flag in ("0", path):
         monkeypatch.setenv("MLXPBD_FLOW", flag)
         if cs:
             monkeypatch.setenv("MLXPBD_FLOW_CS", cs)
@@ -58,7 +60,7 @@ def _resident(sc, steps, graph=True, precision=_lib.MLX_FP32, residuals=False, v
 
 def _same(runs):
     (a, pa), (b, pb) = runs
-    assert "dataflow" in pb and "dataflow" not in pa
+    assert "sweeps, one launch each" in pb and "sweeps, one launch each" not in pa
     for x, y in zip(a, b):
         for u, v in zip(x, y):
             np.testing.assert_array_equal(u, v)
@@ -68,13 +70,14 @@ def _same(runs):
                                                     (STVK, 0.01, "lame")])
 @pytest.mark.parametrize("dims", [(1, 1, 1), (3, 2, 2), (9, 5, 4)])
 @pytest.mark.parametrize("prec", [_lib.MLX_FP32, _lib.MLX_FP64])
-def test_layer_solve(gpu, monkeypatch, energy, alpha1, material, dims, prec):
+@pytest.mark.parametrize("path", ["1", "2"])
+def test_layer_solve(gpu, monkeypatch, energy, alpha1, material, dims, prec, path):
     def make():
         m = block_mesh(dims=dims, energy=energy, seed=5, alpha1=alpha1)
         c = Case(m, [50, 25, 0], [2, 3, 5], seed=6)
         c.integ.boundaryCompliance = 1e-7
         return c, c.product(prec, material)
-    (c, a), (_, b) = _paths(monkeypatch, make)
+    (c, a), (_, b) = _paths(monkeypatch, make, path=path)
     if prec == _lib.MLX_FP32:
         np.testing.assert_array_equal(a[0], b[0])
         np.testing.assert_array_equal(a[4], b[4])
@@ -84,8 +87,10 @@ def test_layer_solve(gpu, monkeypatch, energy, alpha1, material, dims, prec):
 
 @pytest.mark.parametrize("graph", [True, False])
 @pytest.mark.parametrize("residuals", [False, True])
-def test_resident_steps(gpu, monkeypatch, graph, residuals):
-    _same(_paths(monkeypatch, lambda: _resident(scenes.config2(nx=31, ny=13, nz=9), 4, graph, residuals=residuals)))
+@pytest.mark.parametrize("path", ["1", "2"])
+def test_resident_steps(gpu, monkeypatch, graph, residuals, path):
+    _same(_paths(monkeypatch, lambda: _resident(scenes.config2(nx=31, ny=13, nz=9), 4, graph, residuals=residuals),
+                 path=path))
 
 
 @pytest.mark.parametrize("cs", ["1", "2", "16"])
@@ -94,25 +99,26 @@ def test_components(gpu, monkeypatch, cs):
     _same(_paths(monkeypatch, lambda: _resident(scenes.config3(seed=7, n_scenes=9, tmin=600, tmax=6000), 3), cs))
 
 
-@pytest.mark.parametrize("coloring", [False, True])
-@pytest.mark.parametrize("cs", ["1", "4"])
-def test_device_contacts(gpu, monkeypatch, coloring, cs):
+@pytest.mark.parametrize("coloring,path,cs", [(False, "1", "1"), (False, "1", "4"), (True, "1", "1"), (True, "1", "4"),
+                                              (False, "2", "")])
+def test_device_contacts(gpu, monkeypatch, coloring, path, cs):
     """Contacts inside the sweep: after it (the reference's order) and
     coloured with the elastic constraints, below layers with bodies."""
     def make():
         sc = scenes.config4(seed=11, n_boxes=3, cubes=4, grid=(3, 1), spacing=1.5, n_spheres=1, coarse=2, mid=2,
                             drop=(0.005, 0.015), contact_coloring=coloring)
         return _resident(sc, 30, v0z=-1.0)
-    _same(_paths(monkeypatch, make, cs))
+    _same(_paths(monkeypatch, make, cs, path))
 
 
-def test_partial_pins_and_loose_vertices(gpu, monkeypatch):
+@pytest.mark.parametrize("path", ["1", "2"])
+def test_partial_pins(gpu, monkeypatch, path):
     """Pinned DOFs of one axis only, and on a vertex of every corner kind."""
     def make():
         m = block_mesh(dims=(5, 3, 2), energy=NH, seed=9)
         m.pinnedDOFs = np.sort(np.concatenate([m.pinnedDOFs[::2], [3 * m.N - 1]])).astype(np.int32)
         c = Case(m, [0], [4], seed=10)
         return c, c.product(_lib.MLX_FP32)
-    (c, a), (_, b) = _paths(monkeypatch, make)
+    (c, a), (_, b) = _paths(monkeypatch, make, path=path)
     np.testing.assert_array_equal(a[0], b[0])
     np.testing.assert_array_equal(b[0][c.mesh.pinnedDOFs - 1], c.pinnedx.astype(np.float32).astype(np.float64))
