@@ -39,8 +39,11 @@
 // tets 41 / 58 us, 64 scenes of 866 k tets 53 / 95 us.  Polling the records'
 // versions instead of mbarriers measured 33 us on the 27,648 tets (the polls
 // take the shared-memory pipe from the projections), st.async inside the CTA
-// too 45 us on the 98,304 (it goes out to the network and back), bulk copies
-// of the rest data into shared memory no gain.
+// too 45 us on the 98,304 (it goes out to the network and back), the rest data
+// gathered per tet instead of read from chunk planes 58 us on the 98,304.
+// Bulk copies of the rest data into shared memory and prefetches of the next
+// chunk's lines into L1 or L2 gave nothing, two or four smaller CTAs per SM
+// neither.
 //
 // The per-vertex phases of an iteration join the chain: the contacts of a
 // vertex run where their phase falls between two of its tets (before the tet
@@ -62,20 +65,41 @@ template <typename R> __host__ __device__ constexpr int flow_threads() { return 
 constexpr unsigned kFlowFirst = 1, kFlowLast = 2, kFlowPinned = 4, kFlowBefore = 8, kFlowAfter = 16, kFlowFree = 32;
 constexpr int kFlowMaxSlots = 1 << 14, kFlowMaxChunks = 1 << 14;
 
+constexpr int kFlowChunkPins = 64;  // a pinned vertex's last tet is in the chunk
+
 // corner of a tet: x = slot it is read from | corner word << 16, y = where the
 // vertex's next tet reads it: rank << 28 | chunk << 14 | slot
 struct FlowCorner {
   uint2 c[4];
 };
 
+// Rest data of a tet in the chunk planes: DmInv (9), for StVK the corners'
+// inverse masses (4) and the volume, then the material.
+template <int MAT> __host__ __device__ constexpr int flow_planes() {
+  return ((MAT == MAT_NH ? 9 : 14) + mat_stride(MAT) + 3) / 4;
+}
+inline int flow_planes_of(int mat) {
+  switch (mat) {
+    case MAT_NH: return flow_planes<MAT_NH>();
+    case MAT_STVK_ISO: return flow_planes<MAT_STVK_ISO>();
+    case MAT_STVK_BLOCKS: return flow_planes<MAT_STVK_BLOCKS>();
+    default: return flow_planes<MAT_STVK_LAME>();
+  }
+}
+
 template <typename R> struct FlowArgs {
   const int* part_off;      // [G CS + 1] chunks of each part
-  // first position in the list (sorted id if no list); tets; records that
-  // other CTAs send for iteration 0; records that come from this CTA, those of
-  // them that no tet sends for iteration 0 << 16
+  // first position in the list (sorted id if no list); tets, kFlowChunkPins;
+  // records that other CTAs send for iteration 0; records that come from this
+  // CTA, those of them that no tet sends for iteration 0 << 16
   const int4* chunks;
   const int* list;          // layer's elastic tets, NULL = identity
-  const FlowCorner* corner; // [T] sorted ids
+  // per chunk, lane-interleaved planes of 32 vectors: rest data
+  // (flow_planes), corners (2 planes) and vertex ids
+  const R4<R>* rest;
+  const uint4* corner;
+  const int4* vid;
+  R* lambda;                // [chunk][multiplier][32] between the first and the last iteration
   const int* pin_at;        // [3N] index into pin_vals or -1
   const R* pin_vals;
   int* error;
@@ -85,25 +109,35 @@ template <typename R> struct FlowArgs {
   double h, contact_resistance;
 };
 
-__device__ __forceinline__ void flow_push(uint32_t a, uint32_t bar, float4 v) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(a),
-               "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(bar)
-               : "memory");
+// Sends a record to slot address `a` of CTA `to` of the cluster and counts it
+// on the mbarrier at `bar` there: a store and an arrive inside this CTA,
+// st.async and its bytes otherwise (predicated: the lanes of a warp differ,
+// and two branches per corner cost more than the instructions).
+__device__ __forceinline__ void flow_send(uint32_t a, uint32_t bar, unsigned to, unsigned rank, float4 v) {
+  asm volatile(
+      "{.reg .pred l; .reg .b32 ra, rb;\n"
+      "setp.eq.u32 l, %6, %7;\n"
+      "@l st.shared.v4.f32 [%0], {%1, %2, %3, %4};\n"
+      "@l mbarrier.arrive.release.cta.shared::cta.b64 _, [%5], 1;\n"
+      "@!l mapa.shared::cluster.u32 ra, %0, %6;\n"
+      "@!l mapa.shared::cluster.u32 rb, %5, %6;\n"
+      "@!l st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [ra], {%1, %2, %3, %4}, [rb];}" ::"r"(a),
+      "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(bar), "r"(to), "r"(rank)
+      : "memory");
 }
-__device__ __forceinline__ void flow_push(uint32_t a, uint32_t bar, double4 v) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(a),
-               "d"(v.x), "d"(v.y), "r"(bar)
-               : "memory");
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(a + 16),
-               "d"(v.z), "d"(v.w), "r"(bar)
-               : "memory");
-}
-__device__ __forceinline__ void flow_st(uint32_t a, float4 v) {
-  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
-}
-__device__ __forceinline__ void flow_st(uint32_t a, double4 v) {
-  asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v.x), "d"(v.y) : "memory");
-  asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(a + 16), "d"(v.z), "d"(v.w) : "memory");
+__device__ __forceinline__ void flow_send(uint32_t a, uint32_t bar, unsigned to, unsigned rank, double4 v) {
+  asm volatile(
+      "{.reg .pred l; .reg .b32 ra, rb;\n"
+      "setp.eq.u32 l, %6, %7;\n"
+      "@l st.shared.v2.f64 [%0], {%1, %2};\n"
+      "@l st.shared.v2.f64 [%0 + 16], {%3, %4};\n"
+      "@l mbarrier.arrive.release.cta.shared::cta.b64 _, [%5], 1;\n"
+      "@!l mapa.shared::cluster.u32 ra, %0, %6;\n"
+      "@!l mapa.shared::cluster.u32 rb, %5, %6;\n"
+      "@!l st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [ra], {%1, %2}, [rb];\n"
+      "@!l st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [ra + 16], {%3, %4}, [rb];}" ::"r"(a),
+      "d"(v.x), "d"(v.y), "d"(v.z), "d"(v.w), "r"(bar), "r"(to), "r"(rank)
+      : "memory");
 }
 __device__ __forceinline__ void flow_bar_init(uint32_t bar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -161,14 +195,34 @@ template <typename R> struct FlowPos {
   __device__ __forceinline__ void st(int, R4<R> x) const { *p = x; }
 };
 
-// The device-detected elastic contacts of vertex v with record p.
+// The device-detected elastic contacts of the corners marked in m.  One
+// corner of a tet at a time, whichever it is: the lanes of a warp rarely mark
+// more than one, and a pass per corner index would run the projection four
+// times.
 template <typename R>
-__device__ __forceinline__ void flow_contacts(const DevContacts& dc, int v, R4<R>& p, const R4<R>* __restrict__ x0,
-                                              double h, double resistance) {
-  const int i = dc.cidx[v];
-  if (i >= 0) elastic_contacts_of_vertex<R>(dc, i, FlowPos<R>{&p}, x0, h, resistance);
+__device__ __forceinline__ void flow_contacts(const DevContacts& dc, unsigned m, const int (&vk)[4], R4<R> (&p)[4],
+                                              const R4<R>* __restrict__ x0, double h, double resistance) {
+  while (m) {
+    const int k = __ffs(m) - 1;
+    m &= m - 1;
+    const int v = k == 0 ? vk[0] : k == 1 ? vk[1] : k == 2 ? vk[2] : vk[3];
+    const int i = dc.cidx[v];
+    if (i < 0) continue;
+    R4<R> q = k == 0 ? p[0] : k == 1 ? p[1] : k == 2 ? p[2] : p[3];
+    elastic_contacts_of_vertex<R>(dc, i, FlowPos<R>{&q}, x0, h, resistance);
+    if (k == 0) p[0] = q;
+    if (k == 1) p[1] = q;
+    if (k == 2) p[2] = q;
+    if (k == 3) p[3] = q;
+  }
 }
 
+// k_flow_pack of a precision and material: fills the chunk planes.
+const void* flow_pack_kernel_fp32(int mat_kind);
+const void* flow_pack_kernel_fp64(int mat_kind);
+inline const void* flow_pack_kernel(bool fp64, int mat_kind) {
+  return fp64 ? flow_pack_kernel_fp64(mat_kind) : flow_pack_kernel_fp32(mat_kind);
+}
 // k_flow of a precision and material (flow_fp32.cu, flow_fp64.cu); `ct`: with
 // device-detected contacts.
 const void* flow_kernel_fp32(int mat_kind, bool damp, bool ct);

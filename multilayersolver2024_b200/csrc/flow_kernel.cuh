@@ -35,30 +35,84 @@ __global__ void __launch_bounds__(flow_threads<R>(), 1)
     const bool first = it == 0, final = it + 1 == a.iterations;
     for (int j = threadIdx.x >> 5; j < mine; j += nw) {
       const int4 ch = a.chunks[q0 + j];
-      const int n = ch.y;
+      const int n = ch.y & 63;
       const bool active = lane < n;
-      // (the lanes past the end load the chunk's last tet and write nothing)
-      const int i = ch.x + min(lane, n - 1), s = a.list ? a.list[i] : i;
+      // (the planes repeat the chunk's last tet past the end)
+      const size_t q = (size_t)(q0 + j);
+      int s = 0;
+      if (first || final) {
+        const int i = ch.x + min(lane, n - 1);
+        s = a.list ? a.list[i] : i;
+      }
       TetRest<R, MAT> r;
-      load_rest<R, MAT>(td, s, r);
-      const FlowCorner fc = a.corner[s];
+      StvkPre<R> pre;
+      {
+        constexpr int P = flow_planes<MAT>();
+        const R4<R>* rp = a.rest + q * (P * 32) + lane;
+        R w[4 * P];
+#pragma unroll
+        for (int c = 0; c < P; ++c) {
+          const R4<R> v = rp[32 * c];
+          w[4 * c] = v.x; w[4 * c + 1] = v.y; w[4 * c + 2] = v.z; w[4 * c + 3] = v.w;
+        }
+#pragma unroll
+        for (int c = 0; c < 9; ++c) r.G[c] = w[c];
+        constexpr int m0 = MAT == MAT_NH ? 9 : 14;
+#pragma unroll
+        for (int c = 0; c < mat_stride(MAT); ++c) r.mat[c] = w[m0 + c];
+        if constexpr (MAT != MAT_NH) {
+          const R m[4] = {w[9], w[10], w[11], w[12]};
+          r.vol = w[13];
+          stvk_pre<R>(m, r.G, pre);
+        }
+      }
+      FlowCorner fc;
+      {
+        const uint4 c0 = a.corner[q * 64 + lane], c1 = a.corner[q * 64 + 32 + lane];
+        fc.c[0] = make_uint2(c0.x, c0.y);
+        fc.c[1] = make_uint2(c0.z, c0.w);
+        fc.c[2] = make_uint2(c1.x, c1.y);
+        fc.c[3] = make_uint2(c1.z, c1.w);
+      }
+      r.v = make_int4(0, 0, 0, 0);
+      const bool pins = a.pins && (ch.y & kFlowChunkPins);
+      if (first || final || CT || DAMP || pins) r.v = a.vid[q * 32 + lane];
       const int vk[4] = {r.v.x, r.v.y, r.v.z, r.v.w};
+      R* lam = first ? td.lambda + s : a.lambda + q * (32 * num_lambda<MAT>()) + lane;
+      const size_t ls = first ? (size_t)T : 32;
+#pragma unroll
+      for (int l = 0; l < num_lambda<MAT>(); ++l) r.lam[l] = lam[l * ls];
+      // what does not depend on the records: the first tets' positions, and
+      // the pinned values brought close
+      R4<R> p[4];
+      if (first) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (fc.c[k].x & (kFlowFirst << 16)) p[k] = ldcg_r4(pos + vk[k]);
+      }
+      if (pins) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if ((fc.c[k].x & (kFlowLast << 16)) && (fc.c[k].x & (kFlowPinned << 16))) {
+            const int* pa = a.pin_at + 3 * (size_t)vk[k];
+            const int i0 = max(max(pa[0], pa[1]), pa[2]);
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(a.pin_vals + i0));
+          }
+      }
       ok = flow_wait(bars + 8 * j, it & 1, a.error);
       if (!ok) break;
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (!first || !(fc.c[k].x & (kFlowFirst << 16))) p[k] = flow_ld(rec + (fc.c[k].x & 0xffffu) * kRec, R());
       // (no record of the next phase can arrive before this warp's results leave)
       if (lane == 0 && !final) flow_arm(bars + 8 * j, (unsigned)(4 * n - (ch.w & 0xffff)) * kRec);
-      R4<R> p[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if (first && (fc.c[k].x & (kFlowFirst << 16))) p[k] = ldcg_r4(pos + vk[k]);
-        else p[k] = flow_ld(rec + (fc.c[k].x & 0xffffu) * kRec, R());
-      }
       __syncwarp();
       if (active) {
         if (CT) {
+          unsigned m = 0;
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            if (fc.c[k].x & (kFlowBefore << 16)) flow_contacts<R>(dc, vk[k], p[k], oldp, a.h, a.contact_resistance);
+          for (int k = 0; k < 4; ++k) m |= fc.c[k].x & (kFlowBefore << 16) ? 1u << k : 0u;
+          flow_contacts<R>(dc, m, vk, p, oldp, a.h, a.contact_resistance);
         }
         V3<R> X[4];
         R minv[4], lnew[num_lambda<MAT>()];
@@ -67,36 +121,49 @@ __global__ void __launch_bounds__(flow_threads<R>(), 1)
           X[k] = {p[k].x, p[k].y, p[k].z};
           minv[k] = p[k].w;
         }
-        tet_update<R, MAT, DAMP>(r, X, minv, oldp, inv_h2, inv_h, lnew);
+        tet_update<R, MAT, DAMP>(r, X, minv, oldp, inv_h2, inv_h, lnew, &pre);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          p[k] = make_r4<R>(X[k].x, X[k].y, X[k].z, minv[k]);
-          const unsigned word = fc.c[k].x >> 16, to = fc.c[k].y;
-          if (word & kFlowLast) {
-            if (CT && (word & (a.after == 1 ? kFlowFree : kFlowAfter)))
-              flow_contacts<R>(dc, vk[k], p[k], oldp, a.h, a.contact_resistance);
-            if (a.pins && (word & kFlowPinned)) {
+        for (int k = 0; k < 4; ++k) p[k] = make_r4<R>(X[k].x, X[k].y, X[k].z, minv[k]);
+        if (CT) {
+          const unsigned mark = a.after == 1 ? kFlowFree : kFlowAfter;
+          unsigned m = 0;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const unsigned word = fc.c[k].x >> 16;
+            m |= (word & kFlowLast) && (word & mark) ? 1u << k : 0u;
+          }
+          flow_contacts<R>(dc, m, vk, p, oldp, a.h, a.contact_resistance);
+        }
+        if (pins) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if ((fc.c[k].x & (kFlowLast << 16)) && (fc.c[k].x & (kFlowPinned << 16))) {
               // xi(pinnedDOFs) = pinnedx (xpbdLayer3D.m:333)
               const int* pa = a.pin_at + 3 * (size_t)vk[k];
               if (pa[0] >= 0) p[k].x = a.pin_vals[pa[0]];
               if (pa[1] >= 0) p[k].y = a.pin_vals[pa[1]];
               if (pa[2] >= 0) p[k].z = a.pin_vals[pa[2]];
             }
-            if (final) {
-              stcg_r4(pos + vk[k], p[k]);
-              continue;
-            }
+        }
+        if (final) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const unsigned to = fc.c[k].y;
+            if (fc.c[k].x & (kFlowLast << 16)) stcg_r4(pos + vk[k], p[k]);
+            else flow_send(rec + (to & 0x3fffu) * kRec, bars + ((to >> 14) & 0x3fffu) * 8, to >> 28, rank, p[k]);
           }
-          const uint32_t dst = rec + (to & 0x3fffu) * kRec, bar = bars + ((to >> 14) & 0x3fffu) * 8;
-          if ((to >> 28) == rank) {
-            flow_st(dst, p[k]);
-            flow_arrive(bar, 1);
-          } else {
-            flow_push(mapa_rank(dst, to >> 28), mapa_rank(bar, to >> 28), p[k]);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const unsigned to = fc.c[k].y;
+            flow_send(rec + (to & 0x3fffu) * kRec, bars + ((to >> 14) & 0x3fffu) * 8, to >> 28, rank, p[k]);
           }
         }
 #pragma unroll
-        for (int l = 0; l < num_lambda<MAT>(); ++l) td.lambda[(size_t)l * T + s] = lnew[l];
+        for (int l = 0; l < num_lambda<MAT>(); ++l) {
+          if (final) td.lambda[(size_t)l * T + s] = lnew[l];
+          else a.lambda[q * (32 * num_lambda<MAT>()) + 32 * l + lane] = lnew[l];
+        }
       }
       __syncwarp();
     }
@@ -106,9 +173,54 @@ __global__ void __launch_bounds__(flow_threads<R>(), 1)
   cluster_wait();
 }
 
+// The chunk planes of one layer: chunk blockIdx.x, lane threadIdx.x; `corner`
+// by sorted id.
+template <typename R, int MAT>
+__global__ void __launch_bounds__(32) k_flow_pack(TetData<R> td, const int4* __restrict__ chunks,
+                                                  const int* __restrict__ list, const FlowCorner* __restrict__ corner,
+                                                  const double* __restrict__ mass3, R4<R>* __restrict__ rest,
+                                                  uint4* __restrict__ cp, int4* __restrict__ vid) {
+  constexpr int P = flow_planes<MAT>(), m0 = MAT == MAT_NH ? 9 : 14;
+  const int4 ch = chunks[blockIdx.x];
+  const int lane = threadIdx.x, i = ch.x + min(lane, (ch.y & 63) - 1), s = list ? list[i] : i, T = td.T;
+  const size_t q = blockIdx.x;
+  R w[4 * P];
+#pragma unroll
+  for (int c = 0; c < 4 * P; ++c) w[c] = 0;
+  const int4 v = td.vid[s];
+#pragma unroll
+  for (int c = 0; c < 9; ++c) w[c] = td.dminv[(size_t)c * T + s];
+  if constexpr (MAT != MAT_NH) {
+    w[9] = (R)(1.0 / mass3[3 * v.x]);
+    w[10] = (R)(1.0 / mass3[3 * v.y]);
+    w[11] = (R)(1.0 / mass3[3 * v.z]);
+    w[12] = (R)(1.0 / mass3[3 * v.w]);
+    w[13] = td.vol[s];
+  }
+#pragma unroll
+  for (int c = 0; c < mat_stride(MAT); ++c) w[m0 + c] = td.mat[(size_t)c * T + s];
+#pragma unroll
+  for (int c = 0; c < P; ++c)
+    rest[q * (P * 32) + 32 * c + lane] = make_r4<R>(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+  const FlowCorner fc = corner[s];
+  cp[q * 64 + lane] = make_uint4(fc.c[0].x, fc.c[0].y, fc.c[1].x, fc.c[1].y);
+  cp[q * 64 + 32 + lane] = make_uint4(fc.c[2].x, fc.c[2].y, fc.c[3].x, fc.c[3].y);
+  vid[q * 32 + lane] = v;
+}
+
+template <typename R> static const void* flow_pack_kernel_of(int mat_kind) {
+  switch (mat_kind) {
+    case MAT_NH: return (const void*)k_flow_pack<R, MAT_NH>;
+    case MAT_STVK_ISO: return (const void*)k_flow_pack<R, MAT_STVK_ISO>;
+    case MAT_STVK_BLOCKS: return (const void*)k_flow_pack<R, MAT_STVK_BLOCKS>;
+    default: return (const void*)k_flow_pack<R, MAT_STVK_LAME>;
+  }
+}
+
 template <typename R, bool CT> static const void* flow_kernel_of(int mat_kind, bool damp) {
   switch (mat_kind) {
     case MAT_NH: return (const void*)k_flow<R, MAT_NH, false, CT>;
+    case MAT_STVK_ISO: return (const void*)k_flow<R, MAT_STVK_ISO, false, CT>;
     case MAT_STVK_BLOCKS:
       return damp ? (const void*)k_flow<R, MAT_STVK_BLOCKS, true, CT> : (const void*)k_flow<R, MAT_STVK_BLOCKS, false, CT>;
     default:

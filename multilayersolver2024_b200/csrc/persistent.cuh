@@ -111,7 +111,7 @@ template <int MAT> __host__ __device__ constexpr int num_lambda() { return MAT =
 template <typename R, int MAT, bool DAMP>
 __device__ __forceinline__ void tet_update(const TetRest<R, MAT>& r, V3<R> X[4], const R minv[4],
                                            const R4<R>* __restrict__ oldp, R inv_h2, R inv_h,
-                                           R (&lnew)[num_lambda<MAT>()]) {
+                                           R (&lnew)[num_lambda<MAT>()], const StvkPre<R>* pre = nullptr) {
   if constexpr (MAT == MAT_NH) {
     double lam[2] = {(double)r.lam[0], (double)r.lam[1]}, dl[2];
     nh_project<R>(X, minv, r.G, (double)r.mat[0], (double)r.mat[1], (double)inv_h2, lam, dl);
@@ -128,7 +128,8 @@ __device__ __forceinline__ void tet_update(const TetRest<R, MAT>& r, V3<R> X[4],
       Xo[0] = {o0.x, o0.y, o0.z}; Xo[1] = {o1.x, o1.y, o1.z};
       Xo[2] = {o2.x, o2.y, o2.z}; Xo[3] = {o3.x, o3.y, o3.z};
     }
-    stvk_project<R, MAT, DAMP>(X, Xo, minv, r.G, r.vol, cm, r.lam, dl);
+    if (pre) stvk_project<R, MAT, DAMP>(X, Xo, minv, r.G, r.vol, cm, r.lam, dl, *pre);
+    else stvk_project<R, MAT, DAMP>(X, Xo, minv, r.G, r.vol, cm, r.lam, dl);
 #pragma unroll
     for (int q = 0; q < 6; ++q) lnew[q] = r.lam[q] + dl[q];
   }

@@ -226,7 +226,7 @@ struct LayerStatic {
   bool fl_coloured = false;    // the corner words hold the contact phases
   bool fl_list = false;        // with a tet list of its own
   size_t o_fpo = 0, o_fch = 0, o_flist = 0;
-  DevBuf fl_corner;
+  DevBuf fl_rest, fl_corner, fl_vid;  // the chunk planes
   // sweeps through L2 (sweep.cuh): chunks and corner words
   bool sw_ok = false;
   int sw_chunks = 0, sw_D = 0;
@@ -530,11 +530,16 @@ struct Solver final : SolverBase {
   std::vector<int> fl_part;                // [T] part of each sorted tet
   std::vector<ushort4> fl_src;             // [T] slots of its corners
   std::vector<int> vcc_h;                  // contact_coloring: phase of each vertex's contacts
-  DevBuf fl_pin_at;
+  bool fl_iso = false;                     // undamped blocks stored as MAT_STVK_ISO
+  DevBuf fl_pin_at, fl_mat, fl_tmp, fl_lam;
+  int flow_mat() const { return fl_iso ? (int)MAT_STVK_ISO : mat_kind; }
   int plan_flow(const mlx_mesh_desc* md);
   int flow_slots();
   int upload_pin_at();
   int build_flow(LayerStatic& ls, const std::vector<int>& list);
+  const int* flow_list(const LayerStatic& ls, const int* dint) const {
+    return ls.fl_list ? dint + ls.o_flist : (ls.identity_list ? nullptr : dint + ls.o_list);
+  }
   bool flow_layer(const LayerStatic& ls) const { return flow_on && ls.fl_ok && ls.tile.empty(); }
   int launch_flow(const LayerStatic& ls, const int* dint, const mlx_solve_params* P, int iterations, bool pins,
                   const DevContacts& dc, int after);
@@ -1318,7 +1323,18 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
   comp_first.push_back(T);
   int optin = 0;
   CU(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
-  const void* fn[2] = {flow_kernel(sizeof(R) == 8, mat_kind, damp, false), flow_kernel(sizeof(R) == 8, mat_kind, damp, true)};
+  // undamped StVK blocks whose stored (rounded) entries are those of an
+  // isotropic material: three values instead of 24
+  if (mat_kind == MAT_STVK_BLOCKS && !damp) {
+    fl_iso = true;
+    for (int e = 0; e < T && fl_iso; ++e) {
+      const double* al = md->alpha + 36 * (size_t)e;
+      for (int c = 0; c < 3; ++c)
+        for (int r = 0; r < 3; ++r) fl_iso = fl_iso && (R)al[r + 6 * c] == (R)al[r == c ? 0 : 1];
+      for (int q = 4; q < 6; ++q) fl_iso = fl_iso && (R)al[q + 6 * q] == (R)al[3 + 6 * 3];
+    }
+  }
+  const void* fn[2] = {flow_kernel(sizeof(R) == 8, flow_mat(), damp, false), flow_kernel(sizeof(R) == 8, flow_mat(), damp, true)};
   for (const void* f : fn) {
     cudaFuncAttributes fa;
     CU(cudaFuncGetAttributes(&fa, f));
@@ -1434,6 +1450,18 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
     for (int i = best.first[p]; i < best.first[p + 1]; ++i) epart[order.empty() ? i : order[i]] = p;
   fl_part.resize(T);
   for (int s = 0; s < T; ++s) fl_part[s] = epart[s2e[s]];
+  if (fl_iso) {
+    std::vector<R> m3(3 * (size_t)T);
+    for (int s = 0; s < T; ++s) {
+      const double* al = md->alpha + 36 * (size_t)s2e[s];
+      m3[s] = (R)al[0];
+      m3[(size_t)T + s] = (R)al[1];
+      m3[2 * (size_t)T + s] = (R)al[3 + 6 * 3];
+    }
+    CHECK(fl_mat.ensure(sizeof(R) * m3.size()));
+    CU(cudaMemcpyAsync(fl_mat.p, m3.data(), sizeof(R) * m3.size(), cudaMemcpyHostToDevice, stream));
+    CU(cudaStreamSynchronize(stream));
+  }
   return flow_slots();
 }
 
@@ -1634,7 +1662,8 @@ int Solver<R>::build_flow(LayerStatic& ls, const std::vector<int>& clist) {
   for (int d : pinned) pin[d / 3] = 1;
   ls.fl_coloured = !vcc_h.empty();
   std::vector<std::vector<int4>> chunks(P);
-  std::vector<int> first_chunk(N, -1), first_part(N, -1), last_part(N, -1);  // of the vertex's first / latest tet
+  // chunk and part of the vertex's first / latest tet
+  std::vector<int> first_chunk(N, -1), first_part(N, -1), last_chunk(N, -1), last_part(N, -1);
   for (int c = 0; c < C; ++c) {
     const int b = ls.color_start[c], n = ls.color_count[c];
     const int at = ls.identity_list && !ls.fl_list ? color_off[c] : b;
@@ -1668,6 +1697,7 @@ int Solver<R>::build_flow(LayerStatic& ls, const std::vector<int>& clist) {
           }
           last[v[k]] = 4 * s + k;
           last_part[v[k]] = p;
+          last_chunk[v[k]] = j;
           corner[s].c[k] = make_uint2(q[k] | word << 16, 0);
         }
       }
@@ -1684,6 +1714,7 @@ int Solver<R>::build_flow(LayerStatic& ls, const std::vector<int>& clist) {
     }
     uint2& w = corner[last[v] >> 2].c[last[v] & 3];
     w.y = home[v];
+    if (pin[v]) chunks[last_part[v]][last_chunk[v]].y |= kFlowChunkPins;
     // the first tet's record comes from the last one, from iteration 1 on
     if (last_part[v] == first_part[v]) chunks[first_part[v]][first_chunk[v]].w += 1 | 1 << 16;
     w.x |= kFlowLast << 16;
@@ -1708,8 +1739,21 @@ int Solver<R>::build_flow(LayerStatic& ls, const std::vector<int>& clist) {
   while (ls.packed.size() & 3) ls.packed.push_back(0);  // int4 alignment
   ls.o_fch = ls.packed.size();
   ls.packed.insert(ls.packed.end(), flat.begin(), flat.end());
-  CHECK(ls.fl_corner.ensure(sizeof(FlowCorner) * (size_t)T));
-  CU(cudaMemcpyAsync(ls.fl_corner.p, corner.data(), sizeof(FlowCorner) * (size_t)T, cudaMemcpyHostToDevice, stream));
+  // the chunk planes (filled once the packed lists are on the device)
+  const size_t nq = (size_t)std::max(ls.fl_chunks, 1);
+  CHECK(ls.fl_rest.ensure(sizeof(R4<R>) * 32 * nq * flow_planes_of(flow_mat())));
+  CHECK(ls.fl_corner.ensure(sizeof(uint4) * 64 * nq));
+  CHECK(ls.fl_vid.ensure(sizeof(int4) * 32 * nq));
+  // (the resident stepper's and the host calls' layers share the scratch:
+  // it only grows, and a grown one drops the recorded graphs)
+  const size_t lam = sizeof(R) * 32 * nq * (mat_kind == MAT_NH ? 2 : 6);
+  if (fl_lam.bytes < lam) {
+    drop_host_graph();
+    if (sim.graph) { cudaGraphExecDestroy(sim.graph); sim.graph = nullptr; }
+    CHECK(fl_lam.ensure(lam));
+  }
+  CHECK(fl_tmp.ensure(sizeof(FlowCorner) * (size_t)T));
+  CU(cudaMemcpyAsync(fl_tmp.p, corner.data(), sizeof(FlowCorner) * (size_t)T, cudaMemcpyHostToDevice, stream));
   CU(cudaStreamSynchronize(stream));
   ls.fl_ok = true;
   return MLX_OK;
@@ -1722,8 +1766,11 @@ int Solver<R>::launch_flow(const LayerStatic& ls, const int* dint, const mlx_sol
   FlowArgs<R> a;
   a.part_off = dint + ls.o_fpo;
   a.chunks = reinterpret_cast<const int4*>(dint + ls.o_fch);
-  a.list = ls.fl_list ? dint + ls.o_flist : (ls.identity_list ? nullptr : dint + ls.o_list);
-  a.corner = ls.fl_corner.template as<FlowCorner>();
+  a.list = flow_list(ls, dint);
+  a.rest = ls.fl_rest.template as<R4<R>>();
+  a.corner = ls.fl_corner.template as<uint4>();
+  a.vid = ls.fl_vid.template as<int4>();
+  a.lambda = fl_lam.as<R>();
   a.pin_at = fl_pin_at.as<int>();
   a.pin_vals = d_pinx.as<R>();
   a.error = reinterpret_cast<int*>(d_gsync.as<unsigned int>() + 4);
@@ -1753,7 +1800,7 @@ int Solver<R>::launch_flow(const LayerStatic& ls, const int* dint, const mlx_sol
   cfg.numAttrs = 1;
   void* args[] = {&td, &a, &p, &oldp, &inv_h2, &inv_h, &dcv};
   const cudaError_t e =
-      cudaLaunchKernelExC(&cfg, after ? flow_kernel(sizeof(R) == 8, mat_kind, damp, true) : flow_kernel(sizeof(R) == 8, mat_kind, damp, false), args);
+      cudaLaunchKernelExC(&cfg, flow_kernel(sizeof(R) == 8, flow_mat(), damp, after != 0), args);
   if (e != cudaSuccess) return set_error(MLX_ERR_CUDA, std::string("dataflow sweep launch: ") + cudaGetErrorString(e));
   return MLX_OK;
 }
@@ -2091,6 +2138,20 @@ int Solver<R>::build_static(const mlx_layer_desc* ld, int col, LayerStatic& ls, 
   CHECK(ls.dev_rigid.ensure(N));
   CU(cudaMemcpyAsync(ls.dev.p, ls.packed.data(), sizeof(int) * ls.packed.size(), cudaMemcpyHostToDevice, stream));
   CU(cudaMemcpyAsync(ls.dev_rigid.p, isRV, N, cudaMemcpyHostToDevice, stream));
+  if (ls.fl_ok && ls.fl_chunks > 0) {
+    TetData<R> td = tets();
+    if (fl_iso) td.mat = fl_mat.as<R>();
+    const int* dint = ls.dev.as<int>();
+    const int4* ch = reinterpret_cast<const int4*>(dint + ls.o_fch);
+    const int* fl = flow_list(ls, dint);
+    const FlowCorner* cn = fl_tmp.as<FlowCorner>();
+    const double* m3 = d_mass3.as<double>();
+    R4<R>* rest = ls.fl_rest.template as<R4<R>>();
+    uint4* cp = ls.fl_corner.template as<uint4>();
+    int4* vd = ls.fl_vid.template as<int4>();
+    void* args[] = {&td, &ch, &fl, &cn, &m3, &rest, &cp, &vd};
+    CU(cudaLaunchKernel(flow_pack_kernel(sizeof(R) == 8, flow_mat()), dim3(ls.fl_chunks), dim3(32), args, 0, stream));
+  }
   // the host copies above are pageable: make sure they finished before the
   // cached vectors can change
   CU(cudaStreamSynchronize(stream));

@@ -15,10 +15,12 @@ namespace mlx {
 enum MatKind : int {
   MAT_STVK_BLOCKS = 0,  // alpha and alpha*beta blocks, 24 values per tet
   MAT_STVK_LAME = 1,    // mu, lambda, alpha1 -> blocks formed in registers
-  MAT_NH = 2            // 1/(vol mu), 1/(vol (lambda - mu)) or 0 (stable Neo-Hookean D/H pair)
+  MAT_NH = 2,           // 1/(vol mu), 1/(vol (lambda - mu)) or 0 (stable Neo-Hookean D/H pair)
+  MAT_STVK_ISO = 3      // alpha's diagonal, off-diagonal and shear value: undamped blocks whose
+                        // stored entries are equal (every isotropic material's in FP32)
 };
 __host__ __device__ constexpr int mat_stride(int kind) {
-  return kind == MAT_STVK_BLOCKS ? 24 : (kind == MAT_STVK_LAME ? 3 : 2);
+  return kind == MAT_STVK_BLOCKS ? 24 : (kind == MAT_STVK_LAME || kind == MAT_STVK_ISO ? 3 : 2);
 }
 
 template <typename R> struct V3 { R x, y, z; };
@@ -109,6 +111,18 @@ __device__ __forceinline__ void load_compliance(const R* __restrict__ mat, int s
         for (int j = 0; j < 3; ++j) c.gT[i][j] = 0;
       }
     }
+  } else if (MAT == MAT_STVK_ISO) {
+    const R dg = mat[s] * inv_h2, off = mat[(size_t)T + s] * inv_h2, sh = mat[(size_t)2 * T + s] * inv_h2;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      c.aS[i] = sh;
+      c.gS[i] = 0;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        c.aT[i][j] = i == j ? dg : off;
+        c.gT[i][j] = 0;
+      }
+    }
   } else {  // MAT_STVK_LAME: K = [lam+4mu lam lam; ...] (+) 2mu I (Mesh3D.m:449-456)
     R mu = mat[s], lam = mat[(size_t)T + s], a1 = mat[(size_t)2 * T + s];
     R inv4mu = R(1) / (R(4) * mu);
@@ -152,6 +166,37 @@ __device__ __forceinline__ void strain_kin(const V3<R> X[4], const R G[9], Strai
   }
 }
 
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+
+// The part of a projection that does not depend on positions, for callers
+// that wait for the positions: W(i,j) = sum_a minv_a d_a(i) d_a(j).
+template <typename R> struct StvkPre {
+  R W[3][3];
+};
+template <typename R>
+__device__ __forceinline__ void stvk_pre(const R minv[4], const R G[9], StvkPre<R>& p) {
+  R d[4][3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    d[0][i] = G[0 + 3 * i] + G[1 + 3 * i] + G[2 + 3 * i];
+    d[1][i] = -G[0 + 3 * i];
+    d[2][i] = -G[1 + 3 * i];
+    d[3][i] = -G[2 + 3 * i];
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = i; j < 3; ++j) {
+      R s = 0;
+#pragma unroll
+      for (int a = 0; a < 4; ++a) s += minv[a] * d[a][i] * d[a][j];
+      p.W[i][j] = s; p.W[j][i] = s;
+    }
+}
+
 // ---------------------------------------------------------------------------
 // StVK "Voigt" projection of one tet: matStvkVoigtConstraint3D.m:1-22 with the
 // block-decoupled solve of decomposeSolve (:31-45).  Returns dx (in X) and
@@ -159,24 +204,15 @@ __device__ __forceinline__ void strain_kin(const V3<R> X[4], const R G[9], Strai
 template <typename R, int MAT, bool DAMP>
 __device__ __forceinline__ void stvk_project(V3<R> X[4], const V3<R>* Xold, const R minv[4],
                                              const R G[9], R vol, const Compliance<R>& cm,
-                                             const R lam[6], R dl[6]) {
+                                             const R lam[6], R dl[6], const StvkPre<R>& pre) {
   StrainKin<R> k;
   strain_kin<R>(X, G, k);
+  const R (&W)[3][3] = pre.W;
   R FF[3][3];
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int j = i; j < 3; ++j) { FF[i][j] = vdot(k.f[i], k.f[j]); FF[j][i] = FF[i][j]; }
-  R W[3][3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = i; j < 3; ++j) {
-      R s = 0;
-#pragma unroll
-      for (int a = 0; a < 4; ++a) s += minv[a] * k.d[a][i] * k.d[a][j];
-      W[i][j] = s; W[j][i] = s;
-    }
   const R half = R(0.5);
   R C[6] = {vol * (half * FF[0][0] - half), vol * (half * FF[1][1] - half), vol * (half * FF[2][2] - half),
             vol * (half * FF[0][1]), vol * (half * FF[0][2]), vol * (half * FF[1][2])};
@@ -208,16 +244,20 @@ __device__ __forceinline__ void stvk_project(V3<R> X[4], const V3<R>* Xold, cons
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
-    for (int j = 0; j < 3; ++j) GM[i][j] = v2 * W[i][j] * FF[i][j];
+    for (int j = 0; j < 3; ++j) GM[i][j] = DAMP ? v2 * W[i][j] * FF[i][j] : mul_rn(mul_rn(v2, W[i][j]), FF[i][j]);
   R A[3][3], b[3];
 #pragma unroll
   for (int r = 0; r < 3; ++r) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      R s = GM[r][c];
+      if (DAMP) {
+        R s = GM[r][c];
 #pragma unroll
-      for (int q = 0; q < 3; ++q) s += cm.gT[r][q] * GM[q][c];
-      A[r][c] = s + cm.aT[r][c];
+        for (int q = 0; q < 3; ++q) s += cm.gT[r][q] * GM[q][c];
+        A[r][c] = s + cm.aT[r][c];
+      } else {
+        A[r][c] = add_rn(GM[r][c], cm.aT[r][c]);  // (rounded as with a zero gamma)
+      }
     }
     b[r] = -C[r] - (cm.aT[r][0] * lam[0] + cm.aT[r][1] * lam[1] + cm.aT[r][2] * lam[2]) - ng[r];
   }
@@ -242,6 +282,14 @@ __device__ __forceinline__ void stvk_project(V3<R> X[4], const V3<R>* Xold, cons
     X[a].y += s * dx.y;
     X[a].z += s * dx.z;
   }
+}
+
+template <typename R, int MAT, bool DAMP>
+__device__ __forceinline__ void stvk_project(V3<R> X[4], const V3<R>* Xold, const R minv[4], const R G[9], R vol,
+                                             const Compliance<R>& cm, const R lam[6], R dl[6]) {
+  StvkPre<R> pre;
+  stvk_pre<R>(minv, G, pre);
+  stvk_project<R, MAT, DAMP>(X, Xold, minv, G, vol, cm, lam, dl, pre);
 }
 
 // StVK residual terms of one tet (simpleEvaluateAllConstraintResiduals,
