@@ -89,7 +89,7 @@ inline int flow_planes_of(int mat) {
 
 template <typename R> struct FlowArgs {
   const int* part_off;      // [G CS + 1] chunks of each part
-  // first position in the list (sorted id if no list); tets, kFlowChunkPins;
+  // first position in the list (sorted id if no list); tets, kFlowChunkPins, colour << 8;
   // records that other CTAs send for iteration 0; records that come from this
   // CTA, those of them that no tet sends for iteration 0 << 16
   const int4* chunks;

@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(flow_threads<R>(), 1)
       if (lane == 0 && !final) flow_arm(bars + 8 * j, (unsigned)(4 * n - (ch.w & 0xffff)) * kRec);
       __syncwarp();
       if (active) {
-        if (CT) {
+        if (CT && a.after == 2) {
           unsigned m = 0;
 #pragma unroll
           for (int k = 0; k < 4; ++k) m |= fc.c[k].x & (kFlowBefore << 16) ? 1u << k : 0u;
@@ -173,13 +173,11 @@ __global__ void __launch_bounds__(flow_threads<R>(), 1)
   cluster_wait();
 }
 
-// The chunk planes of one layer: chunk blockIdx.x, lane threadIdx.x; `corner`
-// by sorted id.
+// The rest and vertex planes of one layer: chunk blockIdx.x, lane threadIdx.x.
 template <typename R, int MAT>
 __global__ void __launch_bounds__(32) k_flow_pack(TetData<R> td, const int4* __restrict__ chunks,
-                                                  const int* __restrict__ list, const FlowCorner* __restrict__ corner,
-                                                  const double* __restrict__ mass3, R4<R>* __restrict__ rest,
-                                                  uint4* __restrict__ cp, int4* __restrict__ vid) {
+                                                  const int* __restrict__ list, const double* __restrict__ mass3,
+                                                  R4<R>* __restrict__ rest, int4* __restrict__ vid) {
   constexpr int P = flow_planes<MAT>(), m0 = MAT == MAT_NH ? 9 : 14;
   const int4 ch = chunks[blockIdx.x];
   const int lane = threadIdx.x, i = ch.x + min(lane, (ch.y & 63) - 1), s = list ? list[i] : i, T = td.T;
@@ -202,9 +200,6 @@ __global__ void __launch_bounds__(32) k_flow_pack(TetData<R> td, const int4* __r
 #pragma unroll
   for (int c = 0; c < P; ++c)
     rest[q * (P * 32) + 32 * c + lane] = make_r4<R>(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
-  const FlowCorner fc = corner[s];
-  cp[q * 64 + lane] = make_uint4(fc.c[0].x, fc.c[0].y, fc.c[1].x, fc.c[1].y);
-  cp[q * 64 + 32 + lane] = make_uint4(fc.c[2].x, fc.c[2].y, fc.c[3].x, fc.c[3].y);
   vid[q * 32 + lane] = v;
 }
 

@@ -20,7 +20,7 @@ namespace {
 // Breadth-first order of the component containing `start`; returns the
 // last vertex reached.
 int bfs(int start, const std::vector<int>& vt_off, const std::vector<int>& vt, const int32_t* t, int T,
-        std::vector<char>& seen, std::vector<int>& order) {
+        std::vector<char>& seen, std::vector<char>& done, std::vector<int>& order) {
   size_t head = order.size();
   order.push_back(start);
   seen[start] = 1;
@@ -30,6 +30,8 @@ int bfs(int start, const std::vector<int>& vt_off, const std::vector<int>& vt, c
     last = v;
     for (int q = vt_off[v]; q < vt_off[v + 1]; ++q) {
       int e = vt[q];
+      if (done[e]) continue;  // all its corners have been reached
+      done[e] = 1;
       for (int k = 0; k < 4; ++k) {
         int u = t[e + (size_t)T * k] - 1;
         if (!seen[u]) {
@@ -59,12 +61,12 @@ void breadth_first_vertices(int N, int T, const int32_t* t, std::vector<int>& vt
   // breadth-first order, component by component
   order.clear();
   order.reserve(N);
-  std::vector<char> seen(N, 0), probe(N, 0);
+  std::vector<char> seen(N, 0), probe(N, 0), done(T, 0), done_probe(T, 0);
   for (int v0 = 0; v0 < N; ++v0) {
     if (seen[v0]) continue;
     std::vector<int> tmp;
-    int far = bfs(v0, vt_off, vt, t, T, probe, tmp);
-    bfs(far, vt_off, vt, t, T, seen, order);
+    int far = bfs(v0, vt_off, vt, t, T, probe, done_probe, tmp);
+    bfs(far, vt_off, vt, t, T, seen, done, order);
   }
 }
 

@@ -37,7 +37,10 @@
 #include <cstdlib>
 #include <cstdio>
 #include <cstring>
+#include <array>
+#include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -112,6 +115,129 @@ __global__ void k_cast(const double* __restrict__ a, R* __restrict__ out, int n)
 }
 
 inline int blocks_for(long long n, int b) { return (int)((n + b - 1) / b); }
+
+// ---- the vertices' chains of tets, for the one-launch sweeps --------------
+// Corner 4 s + k of sorted tet s and its vertex; sorting by vertex (stable)
+// lists each vertex's corners in colour order.
+static __global__ void k_corner_keys(const int4* __restrict__ vid, int T, int* __restrict__ key, int* __restrict__ val) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= T) return;
+  const int4 v = vid[s];
+  key[4 * s] = v.x; key[4 * s + 1] = v.y; key[4 * s + 2] = v.z; key[4 * s + 3] = v.w;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) val[4 * s + k] = 4 * s + k;
+}
+// off[v] .. off[v + 1]: the corners of vertex v in the sorted list
+static __global__ void k_key_offsets(const int* __restrict__ key, int n, int N, int* __restrict__ off) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i > n) return;
+  const int a = i > 0 ? key[i - 1] : -1, b = i < n ? key[i] : N;
+  for (int v = a + 1; v <= b; ++v) off[v] = i;
+}
+// at[s] = chunk * 32 + lane of the layer's elastic tets
+static __global__ void k_flow_place(const int4* __restrict__ chunks, const int* __restrict__ list, int* __restrict__ at) {
+  const int4 ch = chunks[blockIdx.x];
+  const int lane = threadIdx.x;
+  if (lane < (ch.y & 63)) at[list ? list[ch.x + lane] : ch.x + lane] = blockIdx.x * 32 + lane;
+}
+
+struct FlowLink {
+  const int *voff, *vcor, *at, *part, *part_off;  // chains; chunk * 32 + lane (-1: not elastic) and part of every tet
+  const ushort4* src;      // slots of every tet's corners
+  const int *body, *vcc;   // body of every vertex, contact phase or NULL
+  const int* pin_at;       // [3N] or NULL
+  int4* chunks;            // y: tets | colour << 8
+  uint2* corner;           // the corner planes
+  int* loose;              // [0] a pinned vertex without elastic tet, [1] a vertex of no body without
+  int N, C, cs, bodies;
+};
+// The corner words, the next reader of every record and the chunks' counts:
+// one thread walks one vertex's chain.
+static __global__ void __launch_bounds__(128) k_flow_link(FlowLink a) {
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= a.N) return;
+  const bool pin = a.pin_at && (a.pin_at[3 * v] >= 0 || a.pin_at[3 * v + 1] >= 0 || a.pin_at[3 * v + 2] >= 0);
+  const bool loose = a.body[v] == 0;
+  const unsigned mark = (pin ? kFlowPinned : 0) | (loose ? kFlowFree : 0);
+  const int vcc = a.vcc ? a.vcc[v] : 0;
+  bool taken = false;
+  unsigned word = 0, home = 0;
+  int q0 = -1, p0 = -1, q1 = -1, p1 = -1;  // chunk and part of the first and the latest tet
+  size_t w = 0;                            // the latest corner's place
+  unsigned x = 0;
+  for (int i = a.voff[v]; i < a.voff[v + 1]; ++i) {
+    const int c = a.vcor[i], s = c >> 2, k = c & 3, at = a.at[s];
+    if (at < 0) continue;
+    const int q = at >> 5, lane = at & 31, p = a.part[s];
+    const ushort4 s4 = a.src[s];
+    const unsigned slot = k == 0 ? s4.x : k == 1 ? s4.y : k == 2 ? s4.z : s4.w;
+    const unsigned me = (unsigned)(p % a.cs) << 28 | (unsigned)(q - a.part_off[p]) << 14 | slot;
+    word = mark;
+    if (a.vcc && loose && !taken && (a.chunks[q].y >> 8) > vcc) {
+      taken = true;
+      word |= kFlowBefore;
+    }
+    if (q1 < 0) {
+      home = me;
+      q0 = q;
+      p0 = p;
+      word |= kFlowFirst;
+    } else {
+      a.corner[w] = make_uint2(x, me);
+      atomicAdd(p1 == p ? &a.chunks[q].w : &a.chunks[q].z, 1);
+    }
+    q1 = q;
+    p1 = p;
+    w = ((size_t)q * 64 + (size_t)(k >> 1) * 32 + lane) * 2 + (k & 1);
+    x = slot | word << 16;
+  }
+  if (q1 < 0) {
+    if (pin) a.loose[0] = 1;
+    if (loose) a.loose[1] = 1;
+    return;
+  }
+  word = kFlowLast;
+  // coloured contacts after every tet of this layer; phase C (no free colour)
+  // is the body phase's when the layer has bodies
+  if (a.vcc && loose && !taken && (vcc < a.C || !a.bodies)) word |= kFlowAfter;
+  a.corner[w] = make_uint2(x | word << 16, home);
+  // the first tet's record comes from the last one, from iteration 1 on
+  if (p1 == p0) atomicAdd(&a.chunks[q0].w, 1 | 1 << 16);
+  if (pin) atomicOr(&a.chunks[q1].y, kFlowChunkPins);
+}
+static __global__ void k_scatter_zero(const int* __restrict__ list, int n, int* __restrict__ at) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) at[list[i]] = 0;
+}
+// Corner words of the sweep through L2: the rank of every elastic tet at its
+// vertices; at[s] >= 0 marks the layer's tets, D receives the longest chain.
+static __global__ void __launch_bounds__(128) k_sweep_link(const int* __restrict__ voff, const int* __restrict__ vcor,
+                                                           const int* __restrict__ at, const int* __restrict__ pin_at,
+                                                           int N, unsigned short* __restrict__ corner,
+                                                           int* __restrict__ loose, int* __restrict__ D) {
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= N) return;
+  const bool pin = pin_at && (pin_at[3 * v] >= 0 || pin_at[3 * v + 1] >= 0 || pin_at[3 * v + 2] >= 0);
+  int n = 0, last = -1;
+  for (int i = voff[v]; i < voff[v + 1]; ++i) {
+    const int c = vcor[i];
+    if (at[c >> 2] < 0) continue;
+    corner[c] = (unsigned short)(n++ | (pin ? kSweepPinned : 0));
+    last = c;
+  }
+  if (last >= 0) corner[last] |= kSweepLast;
+  else if (pin) *loose = 1;
+  atomicMax(D, n);
+}
+template <typename R>
+__global__ void k_corner_masses(const int4* __restrict__ vid, const double* __restrict__ mass3, int T,
+                                R4<R>* __restrict__ out) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= T) return;
+  const int4 v = vid[s];
+  out[s] = make_r4<R>((R)(1.0 / mass3[3 * (size_t)v.x]), (R)(1.0 / mass3[3 * (size_t)v.y]),
+                      (R)(1.0 / mass3[3 * (size_t)v.z]), (R)(1.0 / mass3[3 * (size_t)v.w]));
+}
 
 // ---- buffers ---------------------------------------------------------------
 struct DevBuf {
@@ -528,15 +654,17 @@ struct Solver final : SolverBase {
   bool flow_on = false;
   int fl_G = 0, fl_cs = 1, fl_slots = 0, fl_smem = 0;
   std::vector<int> fl_part;                // [T] part of each sorted tet
-  std::vector<ushort4> fl_src;             // [T] slots of its corners
-  std::vector<int> vcc_h;                  // contact_coloring: phase of each vertex's contacts
+  bool fl_reorder = false;                 // the parts are not runs of the element order
+  DevBuf fl_partd, fl_srcd;                // [T] part and corner slots of each sorted tet
+  DevBuf ch_off, ch_cor, fl_at;            // the vertices' chains (corners in colour order), scratch
   bool fl_iso = false;                     // undamped blocks stored as MAT_STVK_ISO
-  DevBuf fl_pin_at, fl_mat, fl_tmp, fl_lam;
+  DevBuf fl_pin_at, fl_mat, fl_lam;
   int flow_mat() const { return fl_iso ? (int)MAT_STVK_ISO : mat_kind; }
   int plan_flow(const mlx_mesh_desc* md);
-  int flow_slots();
   int upload_pin_at();
   int build_flow(LayerStatic& ls, const std::vector<int>& list);
+  int link_flow(LayerStatic& ls);
+  int build_chains();
   const int* flow_list(const LayerStatic& ls, const int* dint) const {
     return ls.fl_list ? dint + ls.o_flist : (ls.identity_list ? nullptr : dint + ls.o_list);
   }
@@ -551,7 +679,8 @@ struct Solver final : SolverBase {
   int sw_sms = 0;
   DevBuf sw_rec, sw_minv, sw_state;
   int plan_sweep();
-  int build_sweep(LayerStatic& ls, const std::vector<int>& list);
+  int build_sweep(LayerStatic& ls);
+  int link_sweep(LayerStatic& ls);
   bool sweep_layer(const LayerStatic& ls, int iterations) const {
     return sweep_on && ls.sw_ok && ls.tile.empty() && (long long)ls.sw_D * std::max(iterations, 1) < kSweepMaxTags;
   }
@@ -780,6 +909,20 @@ int Solver<R>::create(const mlx_mesh_desc* md) {
       mat[(size_t)T + s] = (R)md->lambda[e];
       mat[2 * (size_t)T + s] = (R)(md->alpha1 ? md->alpha1[e] : 0.0);
     }
+  }
+
+  // undamped StVK blocks whose stored (rounded) entries are those of an
+  // isotropic material: three values instead of 24 on the dataflow path
+  if (mat_kind == MAT_STVK_BLOCKS && !damp) {
+    bool iso = true;
+    const size_t n = (size_t)T;
+    for (int q : {4, 8})
+      iso = iso && std::equal(mat.begin(), mat.begin() + n, mat.begin() + q * n);
+    for (int q : {2, 3, 5, 6, 7})
+      iso = iso && std::equal(mat.begin() + n, mat.begin() + 2 * n, mat.begin() + q * n);
+    for (int q : {10, 11})
+      iso = iso && std::equal(mat.begin() + 9 * n, mat.begin() + 10 * n, mat.begin() + q * n);
+    fl_iso = iso;
   }
 
   CU(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
@@ -1277,6 +1420,52 @@ int Solver<R>::launch_groups(const LayerStatic& ls, const int* dint, const mlx_s
   return MLX_OK;
 }
 
+// Shared memory and co-resident clusters of 1, 2, 4, 8 and 16 CTAs of k_flow.
+// The queries take milliseconds and depend on the device and the kernel only,
+// so their results are kept for the process (a few entries, behind a lock).
+struct FlowLimits {
+  int smem = 0, resident[5] = {0, 0, 0, 0, 0};
+};
+static int flow_limits(int device, bool fp64, int mat, bool damp, int threads, FlowLimits& out) {
+  static std::mutex lock;
+  static std::map<std::array<int, 4>, FlowLimits> known;
+  std::lock_guard<std::mutex> g(lock);
+  const std::array<int, 4> key{device, fp64 ? 1 : 0, mat, damp ? 1 : 0};
+  const auto it = known.find(key);
+  if (it != known.end()) {
+    out = it->second;
+    return MLX_OK;
+  }
+  int optin = 0;
+  CU(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+  FlowLimits lim;
+  lim.smem = optin - 1024;
+  for (bool ct : {true, false}) {
+    const void* f = flow_kernel(fp64, mat, damp, ct);
+    CU(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    CU(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, lim.smem));
+    for (int i = 0; i < 5 && !ct; ++i) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(1 << i);
+      cfg.blockDim = dim3(threads);
+      cfg.dynamicSmemBytes = (size_t)lim.smem;
+      cudaLaunchAttribute at;
+      at.id = cudaLaunchAttributeClusterDimension;
+      at.val.clusterDim.x = 1 << i;
+      at.val.clusterDim.y = at.val.clusterDim.z = 1;
+      cfg.attrs = &at;
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&lim.resident[i], f, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        lim.resident[i] = 0;
+      }
+    }
+  }
+  known[key] = lim;
+  out = lim;
+  return MLX_OK;
+}
+
 // Plan of the dataflow path: how many groups of whole components, on clusters
 // of how many CTAs, and the part of every element.
 template <typename R>
@@ -1321,27 +1510,9 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
   }
   const int ncomp = (int)comp_first.size();
   comp_first.push_back(T);
-  int optin = 0;
-  CU(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
-  // undamped StVK blocks whose stored (rounded) entries are those of an
-  // isotropic material: three values instead of 24
-  if (mat_kind == MAT_STVK_BLOCKS && !damp) {
-    fl_iso = true;
-    for (int e = 0; e < T && fl_iso; ++e) {
-      const double* al = md->alpha + 36 * (size_t)e;
-      for (int c = 0; c < 3; ++c)
-        for (int r = 0; r < 3; ++r) fl_iso = fl_iso && (R)al[r + 6 * c] == (R)al[r == c ? 0 : 1];
-      for (int q = 4; q < 6; ++q) fl_iso = fl_iso && (R)al[q + 6 * q] == (R)al[3 + 6 * 3];
-    }
-  }
-  const void* fn[2] = {flow_kernel(sizeof(R) == 8, flow_mat(), damp, false), flow_kernel(sizeof(R) == 8, flow_mat(), damp, true)};
-  for (const void* f : fn) {
-    cudaFuncAttributes fa;
-    CU(cudaFuncGetAttributes(&fa, f));
-    CU(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    fl_smem = optin - 1024 - (int)fa.sharedSizeBytes;  // (the kernels have no static shared memory)
-    CU(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, fl_smem));
-  }
+  FlowLimits lim;
+  CHECK(flow_limits(device, sizeof(R) == 8, flow_mat(), damp, flow_threads<R>(), lim));
+  fl_smem = lim.smem;
   int want_cs = 0;
   if (const char* q = std::getenv("MLXPBD_FLOW_CS")) want_cs = std::atoi(q);
   struct Plan {
@@ -1350,9 +1521,12 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
     long long sum = 0, most = 0;  // vertices summed over the parts, largest part's tets
     double t = -1;
   } best;
-  std::vector<int> stamp(N), order;
-  // vertices of every part of a plan
-  auto count = [&](Plan& pl) {
+  std::vector<int> stamp(N), slot(N), order;
+  std::vector<ushort4> eslot, eslot2;
+  // slots of every element's corners: each part numbers the vertices its
+  // elements touch
+  auto count = [&](Plan& pl, std::vector<ushort4>& out) {
+    out.resize(T);
     std::fill(stamp.begin(), stamp.end(), -1);
     pl.slots = 0;
     pl.sum = 0;
@@ -1360,35 +1534,26 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
       int n = 0;
       for (int i = pl.first[p]; i < pl.first[p + 1]; ++i) {
         const int e = order.empty() ? i : order[i];
+        unsigned short q[4];
         for (int k = 0; k < 4; ++k) {
-          int& s = stamp[md->t[e + (size_t)k * T] - 1];
-          if (s != p) {
-            s = p;
-            ++n;
+          const int v = md->t[e + (size_t)k * T] - 1;
+          if (stamp[v] != p) {
+            stamp[v] = p;
+            slot[v] = n++;
           }
+          q[k] = (unsigned short)slot[v];
         }
+        out[e] = make_ushort4(q[0], q[1], q[2], q[3]);
       }
       pl.slots = std::max(pl.slots, n);
       pl.sum += n;
     }
   };
+  std::vector<Plan> plans;
   for (int cs : {1, 2, 4, 8, 16}) {
     if (want_cs > 0 && cs != want_cs) continue;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(cs);
-    cfg.blockDim = dim3(flow_threads<R>());
-    cfg.dynamicSmemBytes = (size_t)fl_smem;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = cs;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    int resident = 0;
-    if (cudaOccupancyMaxActiveClusters(&resident, fn[0], &cfg) != cudaSuccess || resident < 1) {
-      cudaGetLastError();
-      continue;
-    }
+    const int resident = lim.resident[cs == 1 ? 0 : cs == 2 ? 1 : cs == 4 ? 2 : cs == 8 ? 3 : 4];
+    if (resident < 1) continue;
     Plan pl;
     pl.G = std::min(ncomp, resident);
     pl.cs = cs;
@@ -1416,18 +1581,28 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
     // 393,216 on 16: 112).
     const double chain = 0.9 * C, issue = 0.13 * ((double)pl.most / 32.0 + 0.5 * C);
     pl.t = std::sqrt(chain * chain + issue * issue);
-    if (best.t >= 0 && pl.t >= 0.97 * best.t) continue;
-    count(pl);
-    // barriers: every colour rounds its chunks up in every part
+    plans.push_back(pl);
+  }
+  // the shortest estimate whose slots and chunk barriers (every colour rounds
+  // its chunks up in every part) fit; fewer CTAs where that costs under 3 %
+  std::stable_sort(plans.begin(), plans.end(), [](const Plan& x, const Plan& y) { return x.t < y.t; });
+  for (size_t i = 0; i + 1 < plans.size(); ++i)
+    if (plans[i + 1].cs < plans[i].cs && plans[i + 1].t * 0.97 < plans[i].t) std::swap(plans[i], plans[i + 1]);
+  // (none of them is tried when the sweep through L2 is estimated shorter)
+  const double t_l2 = 1.55 * C + 3.3e-5 * (double)T;
+  for (Plan& pl : plans) {
+    if (!force && pl.t > t_l2) break;
     const long long bars = pl.most / 32 + C;
-    if (pl.slots > kFlowMaxSlots || bars > kFlowMaxChunks || pl.slots * (long long)sizeof(R4<R>) + 8 * bars > fl_smem) continue;
+    if (bars > kFlowMaxChunks) continue;
+    count(pl, eslot);
+    if (pl.slots > kFlowMaxSlots || pl.slots * (long long)sizeof(R4<R>) + 8 * bars > fl_smem) continue;
     best = pl;
+    break;
   }
   // A launch per colour takes ~1.75 us plus its tets' traffic (58 us per sweep
   // of 98 k tets, 85 of 393 k), the sweep through L2 less than that at any
   // size (53 and 62 us).
-  if (!force && (best.t < 0 || best.t > 1.55 * C + 3.3e-5 * (double)T)) return plan_sweep();
-  if (best.t < 0) return MLX_OK;
+  if (best.t < 0) return force ? MLX_OK : plan_sweep();
   if (best.cs > 1 && best.sum > 3 * (long long)N / 2) {
     // parts that share many vertices (an element order of thin slabs): cut
     // the breadth-first order instead where that shares fewer
@@ -1437,71 +1612,75 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
     for (int c = 0; c < ncomp && whole; ++c)
       for (int i = comp_first[c]; i < comp_first[c + 1] && whole; ++i)
         whole = order[i] >= comp_first[c] && order[i] < comp_first[c + 1];
-    if (whole) count(pl);
-    if (whole && pl.sum < best.sum && pl.slots <= best.slots) best = pl;
-    else order.clear();
+    if (whole) count(pl, eslot2);
+    if (whole && pl.sum < best.sum && pl.slots <= best.slots) {
+      best = pl;
+      eslot.swap(eslot2);
+    } else {
+      order.clear();
+    }
   }
   flow_on = true;
+  fl_reorder = !order.empty();
   fl_G = best.G;
   fl_cs = best.cs;
   fl_slots = std::max(best.slots, 1);
+  // a fixed shuffle of the slots spreads a chunk's neighbouring vertices over
+  // the shared-memory banks
+  std::vector<unsigned short> perm(fl_slots);
+  for (int q = 0; q < fl_slots; ++q) perm[q] = (unsigned short)q;
+  for (unsigned q = fl_slots - 1, x = 1; q > 0 && q < (unsigned)fl_slots; --q) {
+    x = x * 1664525u + 1013904223u;
+    std::swap(perm[q], perm[(x >> 8) % (q + 1)]);
+  }
   std::vector<int> epart(T);
   for (int p = 0; p < fl_G * fl_cs; ++p)
     for (int i = best.first[p]; i < best.first[p + 1]; ++i) epart[order.empty() ? i : order[i]] = p;
   fl_part.resize(T);
-  for (int s = 0; s < T; ++s) fl_part[s] = epart[s2e[s]];
-  if (fl_iso) {
-    std::vector<R> m3(3 * (size_t)T);
-    for (int s = 0; s < T; ++s) {
-      const double* al = md->alpha + 36 * (size_t)s2e[s];
-      m3[s] = (R)al[0];
-      m3[(size_t)T + s] = (R)al[1];
-      m3[2 * (size_t)T + s] = (R)al[3 + 6 * 3];
-    }
-    CHECK(fl_mat.ensure(sizeof(R) * m3.size()));
-    CU(cudaMemcpyAsync(fl_mat.p, m3.data(), sizeof(R) * m3.size(), cudaMemcpyHostToDevice, stream));
-    CU(cudaStreamSynchronize(stream));
+  std::vector<ushort4> src(T);
+  for (int s = 0; s < T; ++s) {
+    fl_part[s] = epart[s2e[s]];
+    const ushort4 q = eslot[s2e[s]];
+    src[s] = make_ushort4(perm[q.x], perm[q.y], perm[q.z], perm[q.w]);
   }
-  return flow_slots();
+  CHECK(fl_partd.ensure(sizeof(int) * (size_t)T));
+  CHECK(fl_srcd.ensure(sizeof(ushort4) * (size_t)T));
+  CU(cudaMemcpyAsync(fl_partd.p, fl_part.data(), sizeof(int) * (size_t)T, cudaMemcpyHostToDevice, stream));
+  CU(cudaMemcpyAsync(fl_srcd.p, src.data(), sizeof(ushort4) * (size_t)T, cudaMemcpyHostToDevice, stream));
+  CU(cudaStreamSynchronize(stream));
+  if (fl_iso) {
+    CHECK(fl_mat.ensure(sizeof(R) * 3 * (size_t)T));
+    const int rows[3] = {0, 1, 9};  // alpha's diagonal, off-diagonal and shear entries
+    for (int q = 0; q < 3; ++q)
+      CU(cudaMemcpyAsync(fl_mat.as<R>() + (size_t)q * T, d_mat.as<R>() + (size_t)rows[q] * T, sizeof(R) * T,
+                         cudaMemcpyDeviceToDevice, stream));
+  }
+  return build_chains();
 }
 
-// Slots of the corners of every sorted tet (each part numbers the vertices
-// its tets touch, in an order that spreads neighbours over the shared-memory
-// banks) and the pinned DOFs by vertex.
+// The vertices' chains and the pinned DOFs by vertex.
 template <typename R>
-int Solver<R>::flow_slots() {
-  std::vector<unsigned short> perm(fl_slots);
-  for (int q = 0; q < fl_slots; ++q) perm[q] = (unsigned short)q;
-  for (unsigned q = fl_slots - 1, x = 1; q > 0; --q) {
-    x = x * 1664525u + 1013904223u;
-    std::swap(perm[q], perm[(x >> 8) % (q + 1)]);
-  }
-  const int P = fl_G * fl_cs;
-  std::vector<int> off(P + 1, 0), byp(T), stamp(N, -1), slot(N);
-  for (int s = 0; s < T; ++s) ++off[fl_part[s] + 1];
-  for (int p = 0; p < P; ++p) off[p + 1] += off[p];
-  {
-    std::vector<int> f(off.begin(), off.end() - 1);
-    for (int s = 0; s < T; ++s) byp[f[fl_part[s]]++] = s;
-  }
-  fl_src.assign(T, make_ushort4(0, 0, 0, 0));
-  for (int p = 0; p < P; ++p) {
-    int n = 0;
-    for (int i = off[p]; i < off[p + 1]; ++i) {
-      const int s = byp[i];
-      const int4 v4 = vid_sorted[s];
-      const int v[4] = {v4.x, v4.y, v4.z, v4.w};
-      unsigned short q[4];
-      for (int k = 0; k < 4; ++k) {
-        if (stamp[v[k]] != p) {
-          stamp[v[k]] = p;
-          slot[v[k]] = n++;
-        }
-        q[k] = perm[slot[v[k]]];
-      }
-      fl_src[s] = make_ushort4(q[0], q[1], q[2], q[3]);
-    }
-  }
+int Solver<R>::build_chains() {
+  const int n = 4 * T;
+  int bits = 1;
+  while (bits < 31 && (1 << bits) < N) ++bits;
+  CHECK(ch_cor.ensure(sizeof(int) * (size_t)n));
+  CHECK(ch_off.ensure(sizeof(int) * ((size_t)N + 1)));
+  size_t bytes = 0;
+  int* none = nullptr;
+  CU(cub::DeviceRadixSort::SortPairs(nullptr, bytes, none, none, none, none, n, 0, bits, stream));
+  const size_t arr = (sizeof(int) * (size_t)n + 255) / 256 * 256;
+  DevBuf tmp;  // keys, values, sorted keys, the sort's own
+  CHECK(tmp.ensure(3 * arr + bytes));
+  int* key = tmp.as<int>();
+  int* val = reinterpret_cast<int*>(tmp.as<char>() + arr);
+  int* sorted = reinterpret_cast<int*>(tmp.as<char>() + 2 * arr);
+  k_corner_keys<<<blocks_for(T, 256), 256, 0, stream>>>(d_vid.as<int4>(), T, key, val);
+  CU(cudaGetLastError());
+  CU(cub::DeviceRadixSort::SortPairs(tmp.as<char>() + 3 * arr, bytes, key, sorted, val, ch_cor.as<int>(), n, 0, bits, stream));
+  k_key_offsets<<<blocks_for((long long)n + 1, 256), 256, 0, stream>>>(sorted, n, N, ch_off.as<int>());
+  CU(cudaGetLastError());
+  CU(cudaStreamSynchronize(stream));
   return upload_pin_at();
 }
 
@@ -1529,48 +1708,16 @@ int Solver<R>::plan_sweep() {
   CHECK(sw_state.ensure(sizeof(SweepState)));
   CU(cudaMemsetAsync(sw_rec.p, 0, sizeof(SweepRec<R>) * (size_t)N, stream));
   CU(cudaMemsetAsync(sw_state.p, 0, sizeof(SweepState), stream));
-  std::vector<R4<R>> m4(T);
-  std::vector<R> mi(N);
-  for (int v = 0; v < N; ++v) mi[v] = (R)(1.0 / vmass_h[v]);
-  for (int s = 0; s < T; ++s) {
-    const int4 v = vid_sorted[s];
-    m4[s] = make_r4<R>(mi[v.x], mi[v.y], mi[v.z], mi[v.w]);
-  }
   CHECK(sw_minv.ensure(sizeof(R4<R>) * (size_t)T));
-  CU(cudaMemcpyAsync(sw_minv.p, m4.data(), sizeof(R4<R>) * (size_t)T, cudaMemcpyHostToDevice, stream));
-  CU(cudaStreamSynchronize(stream));
+  k_corner_masses<R><<<blocks_for(T, 256), 256, 0, stream>>>(d_vid.as<int4>(), d_mass3.as<double>(), T, sw_minv.as<R4<R>>());
+  CU(cudaGetLastError());
   sweep_on = true;
-  return upload_pin_at();
+  return build_chains();
 }
 
-// Chunks and corner words of one layer's elastic tets (`list`: their sorted
-// ids in colour order) for the sweep through L2.
+// Chunks of one layer's elastic tets for the sweep through L2.
 template <typename R>
-int Solver<R>::build_sweep(LayerStatic& ls, const std::vector<int>& list) {
-  std::vector<unsigned short> rank(N, 0);
-  std::vector<ushort4> corner(T, make_ushort4(0, 0, 0, 0));
-  for (int s : list) {
-    const int4 v = vid_sorted[s];
-    // (a colour has at most one tet of a vertex, so rank < C)
-    corner[s] = make_ushort4(rank[v.x]++, rank[v.y]++, rank[v.z]++, rank[v.w]++);
-  }
-  std::vector<unsigned char> pin(N, 0);
-  ls.loose_pins = false;
-  for (int d : pinned) {
-    pin[d / 3] = 1;
-    if (rank[d / 3] == 0) ls.loose_pins = true;
-  }
-  ls.sw_D = 1;
-  for (int v = 0; v < N; ++v) ls.sw_D = std::max(ls.sw_D, (int)rank[v]);
-  auto mark = [&](unsigned short& wd, int v) {
-    if (wd + 1 == rank[v]) wd |= kSweepLast;
-    if (pin[v]) wd |= kSweepPinned;
-  };
-  for (int s : list) {
-    const int4 v = vid_sorted[s];
-    ushort4& cw = corner[s];
-    mark(cw.x, v.x); mark(cw.y, v.y); mark(cw.z, v.z); mark(cw.w, v.w);
-  }
+int Solver<R>::build_sweep(LayerStatic& ls) {
   while (ls.packed.size() & 1) ls.packed.push_back(0);  // int2 alignment
   ls.o_swch = ls.packed.size();
   for (int c = 0; c < C; ++c) {
@@ -1582,9 +1729,30 @@ int Solver<R>::build_sweep(LayerStatic& ls, const std::vector<int>& list) {
   }
   ls.sw_chunks = (int)(ls.packed.size() - ls.o_swch) / 2;
   CHECK(ls.sw_corner.ensure(sizeof(ushort4) * (size_t)T));
-  CU(cudaMemcpyAsync(ls.sw_corner.p, corner.data(), sizeof(ushort4) * (size_t)T, cudaMemcpyHostToDevice, stream));
-  CU(cudaStreamSynchronize(stream));
   ls.sw_ok = true;
+  return MLX_OK;
+}
+
+// Its corner words, once the packed lists are on the device.
+template <typename R>
+int Solver<R>::link_sweep(LayerStatic& ls) {
+  CHECK(fl_at.ensure(sizeof(int) * ((size_t)T + 4)));
+  int* at = fl_at.as<int>();
+  const int* dint = ls.dev.as<int>();
+  const int* list = ls.identity_list ? nullptr : dint + ls.o_list;
+  CU(cudaMemsetAsync(at, ls.identity_list ? 0 : 0xff, sizeof(int) * (size_t)T, stream));
+  CU(cudaMemsetAsync(at + T, 0, sizeof(int) * 4, stream));
+  int n = 0;
+  for (int c = 0; c < C; ++c) n += ls.color_count[c];
+  if (list && n > 0) k_scatter_zero<<<blocks_for(n, 256), 256, 0, stream>>>(list, n, at);
+  k_sweep_link<<<blocks_for(N, 128), 128, 0, stream>>>(ch_off.as<int>(), ch_cor.as<int>(), at, fl_pin_at.as<int>(), N,
+                                                       ls.sw_corner.template as<unsigned short>(), at + T, at + T + 1);
+  CU(cudaGetLastError());
+  int* hs = h_scalar.as<int>();
+  CU(cudaMemcpyAsync(hs, at + T, sizeof(int) * 2, cudaMemcpyDeviceToHost, stream));
+  CU(cudaStreamSynchronize(stream));
+  ls.loose_pins = hs[0] != 0;
+  ls.sw_D = std::max(hs[1], 1);
   return MLX_OK;
 }
 
@@ -1637,99 +1805,44 @@ int Solver<R>::build_flow(LayerStatic& ls, const std::vector<int>& clist) {
   const int P = fl_G * fl_cs;
   // the layer's list in (colour, part) order; the sorted order already is
   // that when the parts are runs of the element order
-  std::vector<int> list = clist;
-  ls.fl_list = false;
-  {
+  std::vector<int> own;
+  ls.fl_list = fl_reorder && !clist.empty();
+  if (ls.fl_list) {
+    own.resize(clist.size());
     std::vector<int> at(P + 1);
     for (int c = 0; c < C; ++c) {
       const int b = ls.color_start[c], n = ls.color_count[c];
       std::fill(at.begin(), at.end(), 0);
-      bool run = true;
-      for (int o = 0; o < n; ++o) {
-        ++at[fl_part[clist[b + o]] + 1];
-        run = run && (o == 0 || fl_part[clist[b + o]] >= fl_part[clist[b + o - 1]]);
-      }
-      if (run) continue;
-      ls.fl_list = true;
+      for (int o = 0; o < n; ++o) ++at[fl_part[clist[b + o]] + 1];
       for (int p = 0; p < P; ++p) at[p + 1] += at[p];
-      for (int o = 0; o < n; ++o) list[b + at[fl_part[clist[b + o]]]++] = clist[b + o];
+      for (int o = 0; o < n; ++o) own[b + at[fl_part[clist[b + o]]]++] = clist[b + o];
     }
   }
-  std::vector<FlowCorner> corner(T);
-  std::vector<int> last(N, -1);      // corner (4 s + k) of the vertex's latest tet
-  std::vector<unsigned> home(N, 0);  // where its first tet reads it
-  std::vector<unsigned char> pin(N, 0), taken(N, 0);
-  for (int d : pinned) pin[d / 3] = 1;
-  ls.fl_coloured = !vcc_h.empty();
-  std::vector<std::vector<int4>> chunks(P);
-  // chunk and part of the vertex's first / latest tet
-  std::vector<int> first_chunk(N, -1), first_part(N, -1), last_chunk(N, -1), last_part(N, -1);
+  const std::vector<int>& list = ls.fl_list ? own : clist;
+  // runs of one colour and part, cut into chunks; part by part, colours in order
+  struct Run {
+    int p, at, n, c;
+  };
+  std::vector<Run> runs;
+  std::vector<int> off(P + 1, 0);
   for (int c = 0; c < C; ++c) {
     const int b = ls.color_start[c], n = ls.color_count[c];
     const int at = ls.identity_list && !ls.fl_list ? color_off[c] : b;
     for (int o = 0; o < n;) {
-      const int p = fl_part[list[b + o]], j = (int)chunks[p].size();
-      const unsigned me = (unsigned)(p % fl_cs) << 28 | (unsigned)j << 14;
-      int4 ch = make_int4(at + o, 0, 0, 0);
-      for (; ch.y < 32 && o + ch.y < n && fl_part[list[b + o + ch.y]] == p; ++ch.y) {
-        const int s = list[b + o + ch.y];
-        const int4 v4 = vid_sorted[s];
-        const ushort4 q4 = fl_src[s];
-        const int v[4] = {v4.x, v4.y, v4.z, v4.w};
-        const unsigned q[4] = {q4.x, q4.y, q4.z, q4.w};
-        for (int k = 0; k < 4; ++k) {
-          unsigned word = pin[v[k]] ? kFlowPinned : 0;
-          if (ls.rid[v[k]] == 0) word |= kFlowFree;
-          if (ls.fl_coloured && ls.rid[v[k]] == 0 && !taken[v[k]] && c > vcc_h[v[k]]) {
-            taken[v[k]] = 1;
-            word |= kFlowBefore;
-          }
-          const int l = last[v[k]];
-          if (l >= 0) {
-            corner[l >> 2].c[l & 3].y = me | q[k];
-            if (last_part[v[k]] == p) ++ch.w;
-            else ++ch.z;
-          } else {
-            home[v[k]] = me | q[k];
-            first_chunk[v[k]] = j;
-            first_part[v[k]] = p;
-            word |= kFlowFirst;
-          }
-          last[v[k]] = 4 * s + k;
-          last_part[v[k]] = p;
-          last_chunk[v[k]] = j;
-          corner[s].c[k] = make_uint2(q[k] | word << 16, 0);
-        }
-      }
-      chunks[p].push_back(ch);
-      o += ch.y;
+      const int p = fl_part[list[b + o]];
+      int e = o + 1;
+      while (e < n && fl_part[list[b + e]] == p) ++e;
+      runs.push_back({p, at + o, e - o, c});
+      off[p + 1] += (e - o + 31) / 32;
+      o = e;
     }
   }
-  ls.loose_pins = ls.fl_loose_free = false;
-  for (int v = 0; v < N; ++v) {
-    if (last[v] < 0) {
-      if (pin[v]) ls.loose_pins = true;
-      if (ls.rid[v] == 0) ls.fl_loose_free = true;
-      continue;
-    }
-    uint2& w = corner[last[v] >> 2].c[last[v] & 3];
-    w.y = home[v];
-    if (pin[v]) chunks[last_part[v]][last_chunk[v]].y |= kFlowChunkPins;
-    // the first tet's record comes from the last one, from iteration 1 on
-    if (last_part[v] == first_part[v]) chunks[first_part[v]][first_chunk[v]].w += 1 | 1 << 16;
-    w.x |= kFlowLast << 16;
-    // coloured contacts after every tet of this layer; phase C (no free
-    // colour) is the body phase's when the layer has bodies
-    if (ls.fl_coloured && ls.rid[v] == 0 && !taken[v] && (vcc_h[v] < C || ls.nb == 0)) w.x |= kFlowAfter << 16;
-  }
-  std::vector<int> off(P + 1, 0), flat;
+  ls.fl_max = 0;
   for (int p = 0; p < P; ++p) {
-    off[p + 1] = off[p] + (int)chunks[p].size();
-    for (const int4& ch : chunks[p]) flat.insert(flat.end(), {ch.x, ch.y, ch.z, ch.w});
+    ls.fl_max = std::max(ls.fl_max, off[p + 1]);
+    off[p + 1] += off[p];
   }
   ls.fl_chunks = off[P];
-  ls.fl_max = 0;
-  for (int p = 0; p < P; ++p) ls.fl_max = std::max(ls.fl_max, off[p + 1] - off[p]);
   if ((size_t)fl_slots * sizeof(R4<R>) + 8 * (size_t)ls.fl_max > (size_t)fl_smem || ls.fl_max > kFlowMaxChunks)
     return MLX_OK;
   ls.o_flist = ls.packed.size();
@@ -1738,8 +1851,13 @@ int Solver<R>::build_flow(LayerStatic& ls, const std::vector<int>& clist) {
   ls.packed.insert(ls.packed.end(), off.begin(), off.end());
   while (ls.packed.size() & 3) ls.packed.push_back(0);  // int4 alignment
   ls.o_fch = ls.packed.size();
-  ls.packed.insert(ls.packed.end(), flat.begin(), flat.end());
-  // the chunk planes (filled once the packed lists are on the device)
+  ls.packed.resize(ls.o_fch + 4 * (size_t)ls.fl_chunks, 0);
+  for (const Run& r : runs)
+    for (int o = 0; o < r.n; o += 32) {
+      int* ch = ls.packed.data() + ls.o_fch + 4 * (size_t)off[r.p]++;
+      ch[0] = r.at + o;
+      ch[1] = std::min(32, r.n - o) | r.c << 8;
+    }
   const size_t nq = (size_t)std::max(ls.fl_chunks, 1);
   CHECK(ls.fl_rest.ensure(sizeof(R4<R>) * 32 * nq * flow_planes_of(flow_mat())));
   CHECK(ls.fl_corner.ensure(sizeof(uint4) * 64 * nq));
@@ -1752,10 +1870,62 @@ int Solver<R>::build_flow(LayerStatic& ls, const std::vector<int>& clist) {
     if (sim.graph) { cudaGraphExecDestroy(sim.graph); sim.graph = nullptr; }
     CHECK(fl_lam.ensure(lam));
   }
-  CHECK(fl_tmp.ensure(sizeof(FlowCorner) * (size_t)T));
-  CU(cudaMemcpyAsync(fl_tmp.p, corner.data(), sizeof(FlowCorner) * (size_t)T, cudaMemcpyHostToDevice, stream));
-  CU(cudaStreamSynchronize(stream));
   ls.fl_ok = true;
+  return MLX_OK;
+}
+
+// Fills the layer's chunk planes and counts, once its packed lists are on the
+// device.
+template <typename R>
+int Solver<R>::link_flow(LayerStatic& ls) {
+  ls.loose_pins = ls.fl_loose_free = false;
+  ls.fl_coloured = d_vcc.p != nullptr;
+  CHECK(fl_at.ensure(sizeof(int) * ((size_t)T + 4)));
+  CHECK(h_scalar.ensure(sizeof(double) * 8));
+  int* at = fl_at.as<int>();
+  int* dint = ls.dev.as<int>();
+  int4* ch = reinterpret_cast<int4*>(dint + ls.o_fch);
+  const int* list = flow_list(ls, dint);
+  CU(cudaMemsetAsync(at, 0xff, sizeof(int) * (size_t)T, stream));
+  CU(cudaMemsetAsync(at + T, 0, sizeof(int) * 4, stream));
+  if (ls.fl_chunks > 0) {
+    CU(cudaMemsetAsync(ls.fl_corner.p, 0, sizeof(uint4) * 64 * (size_t)ls.fl_chunks, stream));
+    k_flow_place<<<ls.fl_chunks, 32, 0, stream>>>(ch, list, at);
+  }
+  FlowLink a;
+  a.voff = ch_off.as<int>();
+  a.vcor = ch_cor.as<int>();
+  a.at = at;
+  a.part = fl_partd.as<int>();
+  a.part_off = dint + ls.o_fpo;
+  a.src = fl_srcd.as<ushort4>();
+  a.body = dint + ls.o_vb;
+  a.vcc = ls.fl_coloured ? d_vcc.as<int>() : nullptr;
+  a.pin_at = fl_pin_at.as<int>();
+  a.chunks = ch;
+  a.corner = ls.fl_corner.template as<uint2>();
+  a.loose = at + T;
+  a.N = N;
+  a.C = C;
+  a.cs = fl_cs;
+  a.bodies = ls.nb > 0 ? 1 : 0;
+  k_flow_link<<<blocks_for(N, 128), 128, 0, stream>>>(a);
+  CU(cudaGetLastError());
+  if (ls.fl_chunks > 0) {
+    TetData<R> td = tets();
+    if (fl_iso) td.mat = fl_mat.as<R>();
+    const int4* chc = ch;
+    const double* m3 = d_mass3.as<double>();
+    R4<R>* rest = ls.fl_rest.template as<R4<R>>();
+    int4* vd = ls.fl_vid.template as<int4>();
+    void* args[] = {&td, &chc, &list, &m3, &rest, &vd};
+    CU(cudaLaunchKernel(flow_pack_kernel(sizeof(R) == 8, flow_mat()), dim3(ls.fl_chunks), dim3(32), args, 0, stream));
+  }
+  int* hs = h_scalar.as<int>();
+  CU(cudaMemcpyAsync(hs, at + T, sizeof(int) * 2, cudaMemcpyDeviceToHost, stream));
+  CU(cudaStreamSynchronize(stream));
+  ls.loose_pins = hs[0] != 0;
+  ls.fl_loose_free = hs[1] != 0;
   return MLX_OK;
 }
 
@@ -2103,7 +2273,7 @@ int Solver<R>::build_static(const mlx_layer_desc* ld, int col, LayerStatic& ls, 
   ls.fl_ok = false;
   if (flow_on) CHECK(build_flow(ls, list));
   ls.sw_ok = false;
-  if (sweep_on) CHECK(build_sweep(ls, list));
+  if (sweep_on) CHECK(build_sweep(ls));
   if (cluster_ok) {
     // the elastic list (or the identity) is in sorted order, which is
     // (colour, part) order on the cluster path
@@ -2138,20 +2308,8 @@ int Solver<R>::build_static(const mlx_layer_desc* ld, int col, LayerStatic& ls, 
   CHECK(ls.dev_rigid.ensure(N));
   CU(cudaMemcpyAsync(ls.dev.p, ls.packed.data(), sizeof(int) * ls.packed.size(), cudaMemcpyHostToDevice, stream));
   CU(cudaMemcpyAsync(ls.dev_rigid.p, isRV, N, cudaMemcpyHostToDevice, stream));
-  if (ls.fl_ok && ls.fl_chunks > 0) {
-    TetData<R> td = tets();
-    if (fl_iso) td.mat = fl_mat.as<R>();
-    const int* dint = ls.dev.as<int>();
-    const int4* ch = reinterpret_cast<const int4*>(dint + ls.o_fch);
-    const int* fl = flow_list(ls, dint);
-    const FlowCorner* cn = fl_tmp.as<FlowCorner>();
-    const double* m3 = d_mass3.as<double>();
-    R4<R>* rest = ls.fl_rest.template as<R4<R>>();
-    uint4* cp = ls.fl_corner.template as<uint4>();
-    int4* vd = ls.fl_vid.template as<int4>();
-    void* args[] = {&td, &ch, &fl, &cn, &m3, &rest, &cp, &vd};
-    CU(cudaLaunchKernel(flow_pack_kernel(sizeof(R) == 8, flow_mat()), dim3(ls.fl_chunks), dim3(32), args, 0, stream));
-  }
+  if (ls.fl_ok) CHECK(link_flow(ls));
+  if (ls.sw_ok) CHECK(link_sweep(ls));
   // the host copies above are pageable: make sure they finished before the
   // cached vectors can change
   CU(cudaStreamSynchronize(stream));
@@ -3651,7 +3809,6 @@ int Solver<R>::contact_colours() {
         vcc[v] = c;
         break;
       }
-  vcc_h = vcc;
   CHECK(d_vcc.ensure(sizeof(int) * (size_t)N));
   CHECK(d_cbucket.ensure(sizeof(int) * (size_t)N));
   CHECK(d_coff.ensure(sizeof(int) * (size_t)(C + 2)));
