@@ -195,21 +195,71 @@ template <typename R> struct FlowPos {
   __device__ __forceinline__ void st(int, R4<R> x) const { *p = x; }
 };
 
+// What the contact of one corner does not need the record for, gathered while
+// the warp waits: the chain of loads (index, mask, step-start position,
+// obstacle, multiplier) and the contact's geometry took ~2,000 cycles after
+// the record had arrived.  Covers the tet's first marked corner; k < 0: none,
+// i < 0: no contact, `one`: a single obstacle (n, c, aT and lam hold).
+struct FlowContact {
+  int k, i, f, one;
+  D3 n, c;
+  double aT, lam;
+};
+template <typename R>
+__device__ __forceinline__ FlowContact flow_contact_ahead(const DevContacts& dc, unsigned m, const int (&vk)[4],
+                                                          const R4<R>* __restrict__ x0, double h) {
+  FlowContact a;
+  a.k = -1;
+  a.i = -1;
+  a.f = a.one = 0;
+  a.n = a.c = d3(0, 0, 0);
+  a.aT = a.lam = 0;
+  if (!m) return a;
+  a.k = __ffs(m) - 1;
+  const int v = a.k == 0 ? vk[0] : a.k == 1 ? vk[1] : a.k == 2 ? vk[2] : vk[3];
+  a.i = dc.cidx[v];
+  if (a.i < 0) return a;
+  const unsigned mask = dc.mask[v];
+  const R4<R> s = x0[v];
+  a.f = __ffs(mask) - 1;
+  a.one = (mask & (mask - 1)) == 0;
+  if (!a.one) return a;
+  double comp;
+  obstacle_contact(dc.obs[a.f], (double)s.x, (double)s.y, (double)s.z, a.n, a.c, comp);
+  a.aT = comp / (h * h);
+  a.lam = dc.lambda[(size_t)a.i * dc.nobs + a.f];
+  return a;
+}
+
 // The device-detected elastic contacts of the corners marked in m.  One
 // corner of a tet at a time, whichever it is: the lanes of a warp rarely mark
 // more than one, and a pass per corner index would run the projection four
 // times.
 template <typename R>
-__device__ __forceinline__ void flow_contacts(const DevContacts& dc, unsigned m, const int (&vk)[4], R4<R> (&p)[4],
-                                              const R4<R>* __restrict__ x0, double h, double resistance) {
+__device__ __forceinline__ void flow_contacts(const DevContacts& dc, unsigned m, const FlowContact& a,
+                                              const int (&vk)[4], R4<R> (&p)[4], const R4<R>* __restrict__ x0, double h,
+                                              double resistance) {
   while (m) {
     const int k = __ffs(m) - 1;
     m &= m - 1;
     const int v = k == 0 ? vk[0] : k == 1 ? vk[1] : k == 2 ? vk[2] : vk[3];
-    const int i = dc.cidx[v];
+    const int i = k == a.k ? a.i : dc.cidx[v];
     if (i < 0) continue;
     R4<R> q = k == 0 ? p[0] : k == 1 ? p[1] : k == 2 ? p[2] : p[3];
-    elastic_contacts_of_vertex<R>(dc, i, FlowPos<R>{&q}, x0, h, resistance);
+    if (k == a.k && a.one) {
+      // elastic_contacts_of_vertex with one obstacle
+      const D3 x = d3((double)q.x, (double)q.y, (double)q.z);
+      const double minv = (double)q.w;
+      double phi = dot(a.n, x - a.c);
+      if (phi > 0) phi = 0;
+      const double C = resistance * phi;
+      const double dl = (-C - a.aT * a.lam) / (2 * minv + a.aT);
+      dc.lambda[(size_t)i * dc.nobs + a.f] = a.lam + dl;
+      const D3 xn = d3(x.x + minv * (dl * a.n.x), x.y + minv * (dl * a.n.y), x.z + minv * (dl * a.n.z));
+      q = make_r4<R>((R)xn.x, (R)xn.y, (R)xn.z, q.w);
+    } else {
+      elastic_contacts_of_vertex<R>(dc, i, FlowPos<R>{&q}, x0, h, resistance);
+    }
     if (k == 0) p[0] = q;
     if (k == 1) p[1] = q;
     if (k == 2) p[2] = q;
@@ -224,11 +274,12 @@ inline const void* flow_pack_kernel(bool fp64, int mat_kind) {
   return fp64 ? flow_pack_kernel_fp64(mat_kind) : flow_pack_kernel_fp32(mat_kind);
 }
 // k_flow of a precision and material (flow_fp32.cu, flow_fp64.cu); `ct`: with
-// device-detected contacts.
-const void* flow_kernel_fp32(int mat_kind, bool damp, bool ct);
+// device-detected contacts, `small`: at most 256 threads (FP32: twice the
+// registers, none spilled).
+const void* flow_kernel_fp32(int mat_kind, bool damp, bool ct, bool small);
 const void* flow_kernel_fp64(int mat_kind, bool damp, bool ct);
-inline const void* flow_kernel(bool fp64, int mat_kind, bool damp, bool ct) {
-  return fp64 ? flow_kernel_fp64(mat_kind, damp, ct) : flow_kernel_fp32(mat_kind, damp, ct);
+inline const void* flow_kernel(bool fp64, int mat_kind, bool damp, bool ct, bool small) {
+  return fp64 ? flow_kernel_fp64(mat_kind, damp, ct) : flow_kernel_fp32(mat_kind, damp, ct, small);
 }
 
 }  // namespace mlx

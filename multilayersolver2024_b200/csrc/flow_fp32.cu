@@ -3,8 +3,9 @@
 #include "sweep_kernel.cuh"
 
 namespace mlx {
-const void* flow_kernel_fp32(int mat_kind, bool damp, bool ct) {
-  return ct ? flow_kernel_of<float, true>(mat_kind, damp) : flow_kernel_of<float, false>(mat_kind, damp);
+const void* flow_kernel_fp32(int mat_kind, bool damp, bool ct, bool small) {
+  if (small) return ct ? flow_kernel_of<float, true, 256>(mat_kind, damp) : flow_kernel_of<float, false, 256>(mat_kind, damp);
+  return ct ? flow_kernel_of<float, true, 512>(mat_kind, damp) : flow_kernel_of<float, false, 512>(mat_kind, damp);
 }
 const void* flow_pack_kernel_fp32(int mat_kind) { return flow_pack_kernel_of<float>(mat_kind); }
 const void* sweep_kernel_fp32(int mat_kind, bool damp) { return sweep_kernel_of<float>(mat_kind, damp); }

@@ -9,10 +9,11 @@ namespace mlx {
 // `iterations` sweeps of one layer's elastic tets.  Dynamic shared memory:
 // a.slots records, then an mbarrier per chunk.  CT: with device-detected
 // contacts.
-template <typename R, int MAT, bool DAMP, bool CT>
-__global__ void __launch_bounds__(flow_threads<R>(), 1)
+template <typename R, int MAT, bool DAMP, bool CT, int TH>
+__global__ void __launch_bounds__(TH, 1)
     k_flow(TetData<R> td, FlowArgs<R> a, R4<R>* __restrict__ pos, const R4<R>* __restrict__ oldp, R inv_h2, R inv_h,
            DevContacts dc) {
+  pdl_launch_dependents();
   constexpr uint32_t kRec = sizeof(R4<R>);
   extern __shared__ __align__(16) unsigned char fl_smem[];
   const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -29,6 +30,7 @@ __global__ void __launch_bounds__(flow_threads<R>(), 1)
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   cluster_arrive();
   cluster_wait();
+  pdl_wait();  // (so far only what the layer's build wrote has been read)
   const int T = td.T;
   bool ok = true;
   for (int it = 0; it < a.iterations && ok; ++it) {
@@ -99,6 +101,18 @@ __global__ void __launch_bounds__(flow_threads<R>(), 1)
             asm volatile("prefetch.global.L1 [%0];" ::"l"(a.pin_vals + i0));
           }
       }
+      unsigned mb = 0, ma = 0;  // corners with contacts before / after the projection
+      FlowContact ahead;
+      if (CT) {
+        const unsigned mark = a.after == 1 ? kFlowFree : kFlowAfter;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const unsigned word = fc.c[k].x >> 16;
+          if (a.after == 2 && (word & kFlowBefore)) mb |= 1u << k;
+          if ((word & kFlowLast) && (word & mark)) ma |= 1u << k;
+        }
+        ahead = flow_contact_ahead<R>(dc, active ? mb | ma : 0, vk, oldp, a.h);
+      }
       ok = flow_wait(bars + 8 * j, it & 1, a.error);
       if (!ok) break;
 #pragma unroll
@@ -108,12 +122,7 @@ __global__ void __launch_bounds__(flow_threads<R>(), 1)
       if (lane == 0 && !final) flow_arm(bars + 8 * j, (unsigned)(4 * n - (ch.w & 0xffff)) * kRec);
       __syncwarp();
       if (active) {
-        if (CT && a.after == 2) {
-          unsigned m = 0;
-#pragma unroll
-          for (int k = 0; k < 4; ++k) m |= fc.c[k].x & (kFlowBefore << 16) ? 1u << k : 0u;
-          flow_contacts<R>(dc, m, vk, p, oldp, a.h, a.contact_resistance);
-        }
+        if (CT && mb) flow_contacts<R>(dc, mb, ahead, vk, p, oldp, a.h, a.contact_resistance);
         V3<R> X[4];
         R minv[4], lnew[num_lambda<MAT>()];
 #pragma unroll
@@ -124,16 +133,7 @@ __global__ void __launch_bounds__(flow_threads<R>(), 1)
         tet_update<R, MAT, DAMP>(r, X, minv, oldp, inv_h2, inv_h, lnew, &pre);
 #pragma unroll
         for (int k = 0; k < 4; ++k) p[k] = make_r4<R>(X[k].x, X[k].y, X[k].z, minv[k]);
-        if (CT) {
-          const unsigned mark = a.after == 1 ? kFlowFree : kFlowAfter;
-          unsigned m = 0;
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const unsigned word = fc.c[k].x >> 16;
-            m |= (word & kFlowLast) && (word & mark) ? 1u << k : 0u;
-          }
-          flow_contacts<R>(dc, m, vk, p, oldp, a.h, a.contact_resistance);
-        }
+        if (CT && ma) flow_contacts<R>(dc, ma, ahead, vk, p, oldp, a.h, a.contact_resistance);
         if (pins) {
 #pragma unroll
           for (int k = 0; k < 4; ++k)
@@ -168,9 +168,12 @@ __global__ void __launch_bounds__(flow_threads<R>(), 1)
       __syncwarp();
     }
   }
-  // no CTA leaves while another may still write into its shared memory
+  // no CTA leaves while another may still write into its shared memory: every
+  // record sent was waited for, unless a wait gave up -- then the stores in
+  // flight get time to land once nothing sends any more
   cluster_arrive();
   cluster_wait();
+  if (*reinterpret_cast<volatile int*>(a.error)) __nanosleep(200000);
 }
 
 // The rest and vertex planes of one layer: chunk blockIdx.x, lane threadIdx.x.
@@ -212,14 +215,16 @@ template <typename R> static const void* flow_pack_kernel_of(int mat_kind) {
   }
 }
 
-template <typename R, bool CT> static const void* flow_kernel_of(int mat_kind, bool damp) {
+template <typename R, bool CT, int TH> static const void* flow_kernel_of(int mat_kind, bool damp) {
   switch (mat_kind) {
-    case MAT_NH: return (const void*)k_flow<R, MAT_NH, false, CT>;
-    case MAT_STVK_ISO: return (const void*)k_flow<R, MAT_STVK_ISO, false, CT>;
+    case MAT_NH: return (const void*)k_flow<R, MAT_NH, false, CT, TH>;
+    case MAT_STVK_ISO: return (const void*)k_flow<R, MAT_STVK_ISO, false, CT, TH>;
     case MAT_STVK_BLOCKS:
-      return damp ? (const void*)k_flow<R, MAT_STVK_BLOCKS, true, CT> : (const void*)k_flow<R, MAT_STVK_BLOCKS, false, CT>;
+      return damp ? (const void*)k_flow<R, MAT_STVK_BLOCKS, true, CT, TH>
+                  : (const void*)k_flow<R, MAT_STVK_BLOCKS, false, CT, TH>;
     default:
-      return damp ? (const void*)k_flow<R, MAT_STVK_LAME, true, CT> : (const void*)k_flow<R, MAT_STVK_LAME, false, CT>;
+      return damp ? (const void*)k_flow<R, MAT_STVK_LAME, true, CT, TH>
+                  : (const void*)k_flow<R, MAT_STVK_LAME, false, CT, TH>;
   }
 }
 

@@ -1440,11 +1440,12 @@ static int flow_limits(int device, bool fp64, int mat, bool damp, int threads, F
   CU(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
   FlowLimits lim;
   lim.smem = optin - 1024;
-  for (bool ct : {true, false}) {
-    const void* f = flow_kernel(fp64, mat, damp, ct);
+  for (int v = 3; v >= 0; --v) {
+    const bool ct = v & 1, small = v & 2;
+    const void* f = flow_kernel(fp64, mat, damp, ct, small);
     CU(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     CU(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, lim.smem));
-    for (int i = 0; i < 5 && !ct; ++i) {
+    for (int i = 0; i < 5 && v == 0; ++i) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(1 << i);
       cfg.blockDim = dim3(threads);
@@ -1959,18 +1960,24 @@ int Solver<R>::launch_flow(const LayerStatic& ls, const int* dint, const mlx_sol
   DevContacts dcv = dc;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(fl_G * fl_cs);
-  cfg.blockDim = dim3(32 * std::min(flow_threads<R>() / 32, ls.fl_max));
+  // Eight warps with all the registers they want where a CTA has up to four
+  // chunks per colour (us for 10 sweeps and a step's rest, 512 -> 256 threads:
+  // 32 boxes of 10,368 tets on 4 CTAs each 411 -> 387, 48,384 tets on 16 CTAs
+  // 375 -> 359), sixteen above (98,304 tets 447 -> 498).
+  const bool small = ls.fl_max <= 4 * C;
+  cfg.blockDim = dim3(32 * std::min((small ? 256 : flow_threads<R>()) / 32, ls.fl_max));
   cfg.dynamicSmemBytes = (size_t)fl_slots * sizeof(R4<R>) + 8 * (size_t)ls.fl_max;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = fl_cs;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1] = pdl_attr();  // its barriers are set up while the kernel before it runs
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = pdl ? 2 : 1;
   void* args[] = {&td, &a, &p, &oldp, &inv_h2, &inv_h, &dcv};
   const cudaError_t e =
-      cudaLaunchKernelExC(&cfg, flow_kernel(sizeof(R) == 8, flow_mat(), damp, after != 0), args);
+      cudaLaunchKernelExC(&cfg, flow_kernel(sizeof(R) == 8, flow_mat(), damp, after != 0, small), args);
   if (e != cudaSuccess) return set_error(MLX_ERR_CUDA, std::string("dataflow sweep launch: ") + cudaGetErrorString(e));
   return MLX_OK;
 }
@@ -2526,6 +2533,8 @@ __global__ void __launch_bounds__(256) k_residual_monitor(TetData<R> td, const R
                                                           unsigned* __restrict__ ticket, MonState* ms,
                                                           cudaGraphConditionalHandle loop, int iterations, int is_last,
                                                           MonParams mp, cudaGraphConditionalHandle ns, int ns_every) {
+  pdl_launch_dependents();
+  pdl_wait();
   double acc[1] = {residual_tets<R, MAT>(td, pos, inv_h2, inv_h, inv_h2_d, blockIdx.x * blockDim.x + threadIdx.x,
                                          gridDim.x * blockDim.x)};
   block_sum<1>(acc);
@@ -2917,23 +2926,25 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
         unsigned* ticket = reinterpret_cast<unsigned*>(d_scalar.as<double>() + 7);
         MonState* ms = mon();
         const int its = ld->iterations[layer], il = isLast ? 1 : 0;
+        cudaLaunchConfig_t cfg = pdl_config(tb, 256);
+        cudaLaunchAttribute attr = pdl_attr();
+        cfg.attrs = &attr;
+        cfg.numAttrs = pdl ? 1 : 0;
+        const R4<R>* pc = pos();
+        const double ihd = 1.0 / (h * h);
         switch (mat_kind) {
           case MAT_NH:
-            k_residual_monitor<R, MAT_NH><<<tb, 256, 0, stream>>>(td, pos(), ih2, ih, 1.0 / (h * h), parts, ticket, ms,
-                                                                  h_while_cur, its, il, mp, h_ns,
-                                                                  nsEvery);
+            CU(cudaLaunchKernelEx(&cfg, k_residual_monitor<R, MAT_NH>, td, pc, ih2, ih, ihd, parts, ticket, ms, h_while_cur,
+                                  its, il, mp, h_ns, nsEvery));
             break;
           case MAT_STVK_BLOCKS:
-            k_residual_monitor<R, MAT_STVK_BLOCKS><<<tb, 256, 0, stream>>>(td, pos(), ih2, ih, 1.0 / (h * h), parts,
-                                                                           ticket, ms, h_while_cur, its, il, mp, h_ns,
-                                                                  nsEvery);
+            CU(cudaLaunchKernelEx(&cfg, k_residual_monitor<R, MAT_STVK_BLOCKS>, td, pc, ih2, ih, ihd, parts, ticket, ms,
+                                  h_while_cur, its, il, mp, h_ns, nsEvery));
             break;
           default:
-            k_residual_monitor<R, MAT_STVK_LAME><<<tb, 256, 0, stream>>>(td, pos(), ih2, ih, 1.0 / (h * h), parts,
-                                                                         ticket, ms, h_while_cur, its, il, mp, h_ns,
-                                                                  nsEvery);
+            CU(cudaLaunchKernelEx(&cfg, k_residual_monitor<R, MAT_STVK_LAME>, td, pc, ih2, ih, ihd, parts, ticket, ms,
+                                  h_while_cur, its, il, mp, h_ns, nsEvery));
         }
-        CU(cudaGetLastError());
         ++st.launches;
         CHECK(close_body());
         break;
