@@ -262,6 +262,11 @@ struct DevBuf {
   }
   template <typename T> T* as() const { return static_cast<T*>(p); }
 };
+// a part of a DevBuf
+struct DevPart {
+  char* p = nullptr;
+  template <typename T> T* as() const { return reinterpret_cast<T*>(p); }
+};
 struct PinnedBuf {
   void* p = nullptr;
   size_t bytes = 0;
@@ -352,7 +357,8 @@ struct LayerStatic {
   bool fl_coloured = false;    // the corner words hold the contact phases
   bool fl_list = false;        // with a tet list of its own
   size_t o_fpo = 0, o_fch = 0, o_flist = 0;
-  DevBuf fl_rest, fl_corner, fl_vid;  // the chunk planes
+  DevBuf fl_planes;                   // the chunk planes: rest data, corners, vertex ids
+  size_t o_fcorner = 0, o_fvid = 0;
   // sweeps through L2 (sweep.cuh): chunks and corner words
   bool sw_ok = false;
   int sw_chunks = 0, sw_D = 0;
@@ -655,10 +661,14 @@ struct Solver final : SolverBase {
   int fl_G = 0, fl_cs = 1, fl_slots = 0, fl_smem = 0;
   std::vector<int> fl_part;                // [T] part of each sorted tet
   bool fl_reorder = false;                 // the parts are not runs of the element order
-  DevBuf fl_partd, fl_srcd;                // [T] part and corner slots of each sorted tet
-  DevBuf ch_off, ch_cor, fl_at;            // the vertices' chains (corners in colour order), scratch
+  // per mesh, in one allocation: part and corner slots of each sorted tet, the
+  // vertices' chains (corners in colour order), pinned DOFs by vertex, the
+  // MAT_STVK_ISO values, k_flow_link's scratch
+  DevBuf fl_tables;
+  DevPart fl_partd, fl_srcd, ch_off, ch_cor, fl_pin_at, fl_mat, fl_at;
+  int flow_tables();
   bool fl_iso = false;                     // undamped blocks stored as MAT_STVK_ISO
-  DevBuf fl_pin_at, fl_mat, fl_lam;
+  DevBuf fl_lam;
   int flow_mat() const { return fl_iso ? (int)MAT_STVK_ISO : mat_kind; }
   int plan_flow(const mlx_mesh_desc* md);
   int upload_pin_at();
@@ -1644,13 +1654,11 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
     const ushort4 q = eslot[s2e[s]];
     src[s] = make_ushort4(perm[q.x], perm[q.y], perm[q.z], perm[q.w]);
   }
-  CHECK(fl_partd.ensure(sizeof(int) * (size_t)T));
-  CHECK(fl_srcd.ensure(sizeof(ushort4) * (size_t)T));
+  CHECK(flow_tables());
   CU(cudaMemcpyAsync(fl_partd.p, fl_part.data(), sizeof(int) * (size_t)T, cudaMemcpyHostToDevice, stream));
   CU(cudaMemcpyAsync(fl_srcd.p, src.data(), sizeof(ushort4) * (size_t)T, cudaMemcpyHostToDevice, stream));
   CU(cudaStreamSynchronize(stream));
   if (fl_iso) {
-    CHECK(fl_mat.ensure(sizeof(R) * 3 * (size_t)T));
     const int rows[3] = {0, 1, 9};  // alpha's diagonal, off-diagonal and shear entries
     for (int q = 0; q < 3; ++q)
       CU(cudaMemcpyAsync(fl_mat.as<R>() + (size_t)q * T, d_mat.as<R>() + (size_t)rows[q] * T, sizeof(R) * T,
@@ -1659,14 +1667,33 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
   return build_chains();
 }
 
+template <typename R>
+int Solver<R>::flow_tables() {
+  const size_t t = (size_t)T, n = (size_t)N;
+  size_t used = 0;
+  struct Part {
+    DevPart* t;
+    size_t bytes;
+  } parts[] = {{&fl_partd, sizeof(int) * t},       {&fl_srcd, sizeof(ushort4) * t},
+               {&ch_cor, sizeof(int) * 4 * t},     {&ch_off, sizeof(int) * (n + 1)},
+               {&fl_at, sizeof(int) * (t + 4)},    {&fl_pin_at, pinned.empty() ? 0 : sizeof(int) * 3 * n},
+               {&fl_mat, fl_iso ? sizeof(R) * 3 * t : 0}};
+  for (const Part& q : parts) used += (q.bytes + 255) / 256 * 256;
+  CHECK(fl_tables.ensure(used));
+  used = 0;
+  for (const Part& q : parts) {
+    q.t->p = q.bytes ? fl_tables.as<char>() + used : nullptr;
+    used += (q.bytes + 255) / 256 * 256;
+  }
+  return MLX_OK;
+}
+
 // The vertices' chains and the pinned DOFs by vertex.
 template <typename R>
 int Solver<R>::build_chains() {
   const int n = 4 * T;
   int bits = 1;
   while (bits < 31 && (1 << bits) < N) ++bits;
-  CHECK(ch_cor.ensure(sizeof(int) * (size_t)n));
-  CHECK(ch_off.ensure(sizeof(int) * ((size_t)N + 1)));
   size_t bytes = 0;
   int* none = nullptr;
   CU(cub::DeviceRadixSort::SortPairs(nullptr, bytes, none, none, none, none, n, 0, bits, stream));
@@ -1690,7 +1717,6 @@ int Solver<R>::upload_pin_at() {
   if (pinned.empty()) return MLX_OK;
   std::vector<int> at(3 * (size_t)N, -1);
   for (size_t i = 0; i < pinned.size(); ++i) at[pinned[i]] = (int)i;
-  CHECK(fl_pin_at.ensure(sizeof(int) * at.size()));
   CU(cudaMemcpyAsync(fl_pin_at.p, at.data(), sizeof(int) * at.size(), cudaMemcpyHostToDevice, stream));
   CU(cudaStreamSynchronize(stream));
   return MLX_OK;
@@ -1705,6 +1731,7 @@ int Solver<R>::plan_sweep() {
   CU(cudaDeviceGetAttribute(&sw_sms, cudaDevAttrMultiProcessorCount, device));
   CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sweep_kernel(sizeof(R) == 8, mat_kind, damp), kSweepThreads, 0));
   if (per_sm < 1) return MLX_OK;
+  CHECK(flow_tables());
   CHECK(sw_rec.ensure(sizeof(SweepRec<R>) * (size_t)N));
   CHECK(sw_state.ensure(sizeof(SweepState)));
   CU(cudaMemsetAsync(sw_rec.p, 0, sizeof(SweepRec<R>) * (size_t)N, stream));
@@ -1737,7 +1764,6 @@ int Solver<R>::build_sweep(LayerStatic& ls) {
 // Its corner words, once the packed lists are on the device.
 template <typename R>
 int Solver<R>::link_sweep(LayerStatic& ls) {
-  CHECK(fl_at.ensure(sizeof(int) * ((size_t)T + 4)));
   int* at = fl_at.as<int>();
   const int* dint = ls.dev.as<int>();
   const int* list = ls.identity_list ? nullptr : dint + ls.o_list;
@@ -1860,9 +1886,9 @@ int Solver<R>::build_flow(LayerStatic& ls, const std::vector<int>& clist) {
       ch[1] = std::min(32, r.n - o) | r.c << 8;
     }
   const size_t nq = (size_t)std::max(ls.fl_chunks, 1);
-  CHECK(ls.fl_rest.ensure(sizeof(R4<R>) * 32 * nq * flow_planes_of(flow_mat())));
-  CHECK(ls.fl_corner.ensure(sizeof(uint4) * 64 * nq));
-  CHECK(ls.fl_vid.ensure(sizeof(int4) * 32 * nq));
+  ls.o_fcorner = sizeof(R4<R>) * 32 * nq * flow_planes_of(flow_mat());
+  ls.o_fvid = ls.o_fcorner + sizeof(uint4) * 64 * nq;
+  CHECK(ls.fl_planes.ensure(ls.o_fvid + sizeof(int4) * 32 * nq));
   // (the resident stepper's and the host calls' layers share the scratch:
   // it only grows, and a grown one drops the recorded graphs)
   const size_t lam = sizeof(R) * 32 * nq * (mat_kind == MAT_NH ? 2 : 6);
@@ -1881,7 +1907,6 @@ template <typename R>
 int Solver<R>::link_flow(LayerStatic& ls) {
   ls.loose_pins = ls.fl_loose_free = false;
   ls.fl_coloured = d_vcc.p != nullptr;
-  CHECK(fl_at.ensure(sizeof(int) * ((size_t)T + 4)));
   CHECK(h_scalar.ensure(sizeof(double) * 8));
   int* at = fl_at.as<int>();
   int* dint = ls.dev.as<int>();
@@ -1890,7 +1915,7 @@ int Solver<R>::link_flow(LayerStatic& ls) {
   CU(cudaMemsetAsync(at, 0xff, sizeof(int) * (size_t)T, stream));
   CU(cudaMemsetAsync(at + T, 0, sizeof(int) * 4, stream));
   if (ls.fl_chunks > 0) {
-    CU(cudaMemsetAsync(ls.fl_corner.p, 0, sizeof(uint4) * 64 * (size_t)ls.fl_chunks, stream));
+    CU(cudaMemsetAsync(ls.fl_planes.template as<char>() + ls.o_fcorner, 0, sizeof(uint4) * 64 * (size_t)ls.fl_chunks, stream));
     k_flow_place<<<ls.fl_chunks, 32, 0, stream>>>(ch, list, at);
   }
   FlowLink a;
@@ -1904,7 +1929,7 @@ int Solver<R>::link_flow(LayerStatic& ls) {
   a.vcc = ls.fl_coloured ? d_vcc.as<int>() : nullptr;
   a.pin_at = fl_pin_at.as<int>();
   a.chunks = ch;
-  a.corner = ls.fl_corner.template as<uint2>();
+  a.corner = reinterpret_cast<uint2*>(ls.fl_planes.template as<char>() + ls.o_fcorner);
   a.loose = at + T;
   a.N = N;
   a.C = C;
@@ -1917,8 +1942,8 @@ int Solver<R>::link_flow(LayerStatic& ls) {
     if (fl_iso) td.mat = fl_mat.as<R>();
     const int4* chc = ch;
     const double* m3 = d_mass3.as<double>();
-    R4<R>* rest = ls.fl_rest.template as<R4<R>>();
-    int4* vd = ls.fl_vid.template as<int4>();
+    R4<R>* rest = ls.fl_planes.template as<R4<R>>();
+    int4* vd = reinterpret_cast<int4*>(ls.fl_planes.template as<char>() + ls.o_fvid);
     void* args[] = {&td, &chc, &list, &m3, &rest, &vd};
     CU(cudaLaunchKernel(flow_pack_kernel(sizeof(R) == 8, flow_mat()), dim3(ls.fl_chunks), dim3(32), args, 0, stream));
   }
@@ -1938,9 +1963,9 @@ int Solver<R>::launch_flow(const LayerStatic& ls, const int* dint, const mlx_sol
   a.part_off = dint + ls.o_fpo;
   a.chunks = reinterpret_cast<const int4*>(dint + ls.o_fch);
   a.list = flow_list(ls, dint);
-  a.rest = ls.fl_rest.template as<R4<R>>();
-  a.corner = ls.fl_corner.template as<uint4>();
-  a.vid = ls.fl_vid.template as<int4>();
+  a.rest = ls.fl_planes.template as<R4<R>>();
+  a.corner = reinterpret_cast<const uint4*>(ls.fl_planes.template as<char>() + ls.o_fcorner);
+  a.vid = reinterpret_cast<const int4*>(ls.fl_planes.template as<char>() + ls.o_fvid);
   a.lambda = fl_lam.as<R>();
   a.pin_at = fl_pin_at.as<int>();
   a.pin_vals = d_pinx.as<R>();
@@ -2815,7 +2840,12 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
     const bool flow = flow_layer(ls) && (!flowDev || (!ls.fl_loose_free && (!dc.colored || ls.fl_coloured)));
     const int flowAfter = !flowDev ? 0 : (dc.colored ? 2 : 1);
     const int iters = std::max(ld->iterations[layer], 0);
-    const bool sweep = !dc.colored && sweep_layer(ls, P->compute_residuals ? 1 : iters);
+    // (a loop whose stop rules run on the host synchronises after every
+    // iteration, where a cooperative launch costs more than the sweep saves:
+    // 393 k tets with the PCG to residual 1e-4, 56.6 ms with the colour
+    // launches and 66.4 with it)
+    const bool hostRules = P->compute_residuals && !devmon;
+    const bool sweep = !dc.colored && !hostRules && sweep_layer(ls, P->compute_residuals ? 1 : iters);
     // nothing but the sweep, its contacts and the pins
     const bool flowAll = ls.nb == 0 && nK == 0 && (flow || (sweep && !dc.nobs));
     if (flowAll && !P->compute_residuals) {
