@@ -599,6 +599,11 @@ def run_ours(args, rank, world, local):
         peak, peak_kind = measured_peak_hbm()
         if solver_launch_path.startswith("cluster"):
             sweep_kernel = "k_layer_cluster (whole projectGS loop of a layer)"
+        elif solver_launch_path.startswith("dataflow"):
+            sweep_kernel = ("k_flow (body-free layers: the whole projectGS loop in one launch, vertex records in shared "
+                            "memory; layers with bodies: one launch per sweep)")
+        elif solver_launch_path.startswith("version-ordered"):
+            sweep_kernel = "k_sweep (all colours of a sweep in one launch, vertex records through L2)"
         elif "CTAs each owning whole components" in solver_launch_path:
             sweep_kernel = ("k_layer_groups (whole projectGS loop of each body-free layer; algorithmic bytes without "
                             "vertex records, which stay in shared memory) + k_project_color (layers with bodies)")
@@ -609,7 +614,7 @@ def run_ours(args, rank, world, local):
         if groups_only and profiled_dram_bytes_per_tet("k_layer_groups") is not None:
             # one launch = the whole projectGS loop of the layer: T x iterations projections
             traffic = profiled_dram_bytes_per_tet("k_layer_groups") * m.T * sum(sc.iterations)
-        elif profiled_dram_bytes_per_tet() is not None:
+        elif sweep_kernel.startswith("k_project_color") and profiled_dram_bytes_per_tet() is not None:
             traffic = (profiled_dram_bytes_per_tet() * sweep_bytes / solver_bytes_per_tet(m, MLX_FP32)
                        / max(sweep_launches, 1))
         else:
