@@ -604,8 +604,9 @@ struct Solver final : SolverBase {
   PinnedBuf h_gsync;
   PinnedBuf h_mon;  // the device monitor's state, staged for a layer solve replayed as a graph
   long long last_launches = 0;
-  // Fixed-iteration layers run as one launch per colour, each launched as a
-  // programmatic dependent of the previous (off with MLXPBD_PDL=0).  The
+  // Layers that neither the dataflow sweeps nor the sweeps through L2 (below)
+  // take run as one launch per colour, each launched as a programmatic
+  // dependent of the previous (MLXPBD_PDL=0: an ordinary launch).  The
   // persistent one-launch-per-layer kernel (MLXPBD_PERSISTENT=1; one CTA of
   // 128 threads per SM unless MLXPBD_PERSIST_CTAS says otherwise) is kept as
   // an option: on B200 its grid barrier costs more than a dependent launch.
@@ -618,7 +619,8 @@ struct Solver final : SolverBase {
   // fixed-iteration layers run as one cluster launch each when the vertex
   // records of the mesh fit in the shared memory of a cluster
   // (MLXPBD_CLUSTER_SIZE forces the number of CTAs, a power of two up to 16).
-  // Off by default: on a 98k-tet mesh one launch per colour is faster.
+  // Off by default: on a 98k-tet mesh one launch per colour is faster, the
+  // dataflow sweep more so.
   bool cluster_ok = false;
   int cl_size = 0, cl_threads = 0, cl_rec_slots = 0, cl_lam_slots = 0;
   size_t cl_smem = 0;
@@ -633,7 +635,13 @@ struct Solver final : SolverBase {
   // Chosen at mlx_create when the components are contiguous vertex and tet
   // ranges, every group fits in a CTA's shared memory and the estimated sweep
   // is shorter than with colour launches; MLXPBD_GROUPS=0 turns it off, =1
-  // skips the estimate.
+  // skips the estimate.  Beside the dataflow sweeps they keep the body-free
+  // layers with device-detected contacts in the reference's order (after every
+  // sweep): a thread per contact here, while there a vertex's contact holds up
+  // its tets' next sweep.  Resting boxes, 4 steps here / there: 6 of 750 tets
+  // 3.2 / 3.4 ms, 32 of 3,072 3.8 / 4.9, 32 of 10,368 5.6 / 5.9 (with few
+  // contacts 5.5 / 5.0); contacts coloured with the tets 3.9 / 3.2, 5.2 / 4.2,
+  // 7.9 / 5.3, and without contacts 70 / 39 us per sweep of the largest.
   bool groups_ok = false;
   int gr_G = 0;
   int gr_cs = 1;  // CTAs per group (a thread-block cluster when > 1)
@@ -670,6 +678,7 @@ struct Solver final : SolverBase {
   bool fl_iso = false;                     // undamped blocks stored as MAT_STVK_ISO
   DevBuf fl_lam;
   int flow_mat() const { return fl_iso ? (int)MAT_STVK_ISO : mat_kind; }
+  bool flow_forced = false;  // MLXPBD_FLOW=1: no other path beside it
   int plan_flow(const mlx_mesh_desc* md);
   int upload_pin_at();
   int build_flow(LayerStatic& ls, const std::vector<int>& list);
@@ -740,11 +749,11 @@ struct Solver final : SolverBase {
   long long sim_launches_per_step() const override { return sim.launches_per_step; }
   std::string launch_path() const override {
     if (persistent) return "persistent cooperative kernel per layer (" + std::to_string(persist_ctas) + " CTAs)";
-    if (groups_ok && !cluster_ok && gr_cs > 1)
+    if (groups_ok && !cluster_ok && !flow_on && gr_cs > 1)
       return "body-free layers: one launch, " + std::to_string(gr_G) + " clusters of " + std::to_string(gr_cs) +
              " CTAs each owning whole components (records in distributed shared memory); other layers: one launch "
              "per colour (programmatic dependent launches)";
-    if (groups_ok && !cluster_ok)
+    if (groups_ok && !cluster_ok && !flow_on)
       return "body-free layers: one launch, " + std::to_string(gr_G) + " CTAs each owning whole components "
              "(records in shared memory); other layers: one launch per colour (programmatic dependent launches)";
     if (cluster_ok)
@@ -981,7 +990,7 @@ int Solver<R>::create(const mlx_mesh_desc* md) {
   vid_sorted = vid;
   if (cluster_ok) vowner = mp.vowner;
   CHECK(plan_flow(md));
-  if (!flow_on && !sweep_on) CHECK(plan_groups(md));
+  if (!sweep_on && !flow_forced) CHECK(plan_groups(md));
   if (md->mu && md->lambda) {
     pcg_G.resize(9 * (size_t)T);
     pcg_vol.resize(T);
@@ -1482,7 +1491,7 @@ static int flow_limits(int device, bool fp64, int mat, bool damp, int threads, F
 template <typename R>
 int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
   const char* env = std::getenv("MLXPBD_FLOW");
-  const bool force = env && std::string(env) == "1";
+  const bool force = flow_forced = env && std::string(env) == "1";
   if ((env && std::string(env) == "0") || persistent || cluster_ok || std::getenv("MLXPBD_PDL")) return MLX_OK;
   if (env && std::string(env) == "2") return plan_sweep();
   if (!force && std::getenv("MLXPBD_GROUPS")) return MLX_OK;
@@ -2812,7 +2821,8 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
       }
       continue;
     }
-    if (groups_ok && ls.gr_ok && ls.nb == 0 && !P->compute_residuals && (gr_cs == 1 || (!dc.nobs && nK == 0))) {
+    if (groups_ok && ls.gr_ok && ls.nb == 0 && !P->compute_residuals && (gr_cs == 1 || (!dc.nobs && nK == 0)) &&
+        (!flow_layer(ls) || (dc.nobs > 0 && !dc.colored))) {
       // a body-free layer with a fixed iteration count: one launch, a CTA per
       // group of components
       const int iters = std::max(ld->iterations[layer], 0);

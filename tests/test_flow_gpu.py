@@ -111,6 +111,25 @@ def test_device_contacts(gpu, monkeypatch, coloring, path, cs):
     _same(_paths(monkeypatch, make, cs, path))
 
 
+@pytest.mark.parametrize("coloring", [False, True])
+@pytest.mark.parametrize("boxes,cubes", [(2, 2), (6, 5)])
+def test_device_contacts_default(gpu, monkeypatch, boxes, cubes, coloring):
+    """The paths picked without switches: reference-order contacts of
+    body-free layers on the component groups where those are planned, the
+    rest on the dataflow sweeps; the same bits as with the
+    colour launches."""
+    def make():
+        sc = scenes.config4(seed=12, n_boxes=boxes, cubes=cubes, grid=(boxes, 1), spacing=1.5, n_spheres=1, coarse=2,
+                            mid=2, drop=(0.005, 0.015), contact_coloring=coloring)
+        return _resident(sc, 30, v0z=-1.0)
+    monkeypatch.setenv("MLXPBD_FLOW", "0")
+    monkeypatch.setenv("MLXPBD_GROUPS", "0")
+    a = make()
+    monkeypatch.delenv("MLXPBD_FLOW")
+    monkeypatch.delenv("MLXPBD_GROUPS")
+    _same([a, make()])
+
+
 @pytest.mark.parametrize("path", ["1", "2"])
 def test_partial_pins(gpu, monkeypatch, path):
     """Pinned DOFs of one axis only, and on a vertex of every corner kind."""
