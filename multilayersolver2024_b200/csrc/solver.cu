@@ -2795,25 +2795,40 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
     const int ecBlocks = dc.nobs ? std::max(1, std::min(blocks_for(N, kBodyThreads), 296))
                                  : blocks_for(L.n_ec_groups, kBodyThreads);
     bool stopSolve = false;
-    if ((persistent || (cluster_ok && ls.cl_ok)) && !P->compute_residuals && !dc.nobs) {
-      // fixed iteration count: the whole projectGS loop of the layer in one launch
-      const int iters = std::max(ld->iterations[layer], 0);
-      if (iters > 0) {
+    const int iters = std::max(ld->iterations[layer], 0);
+    // A fixed number of iterations whose loop is in the launch: one launch, or
+    // one per correction interval.  `bytes`: of one iteration, `once`: of a launch.
+    const int interval = nsLayer && ns_every > 0 ? ns_every : std::max(iters, 1);
+    auto fixed_loop = [&](double bytes, double once, auto&& launch) -> int {
+      for (int done = 0; done < iters; done += interval) {
+        const int n = std::min(interval, iters - done);
+        if (done > 0) CHECK(ns_correct(h, &st.launches));
         const bool timed = sweep_timing && tev_used + 2 <= tev.size();
         if (timed) CHECK(record_event(tev[tev_used], capturing));
-        if (persistent) CHECK(launch_persistent(ls, dint, L, cd, P, iters, bodyWork, w));
-        else CHECK(launch_cluster(ls, dint, L, cd, P, iters, bodyWork, w));
+        CHECK(launch(n));
         if (timed) {
-          double b = 0;
-          for (int c = 0; c < C; ++c) b += ls.color_count[c] * (bytes_per_tet() + (ls.identity_list ? 0.0 : 4.0));
           CHECK(record_event(tev[tev_used + 1], capturing));
-          tev_bytes[tev_used / 2] = b * iters;
+          tev_bytes[tev_used / 2] = bytes * n + once;
           tev_launches[tev_used / 2] = 1;
           tev_used += 2;
         }
         ++st.launches;
-        st.totalIterations += iters;
+        st.totalIterations += n;
       }
+      return MLX_OK;
+    };
+    auto sweep_bytes_of = [&](double per_tet) {
+      double b = 0;
+      for (int c = 0; c < C; ++c) b += ls.color_count[c] * (per_tet + (ls.identity_list ? 0.0 : 4.0));
+      return b;
+    };
+    const double records_once = 2.0 * (double)N * sizeof(R4<R>);  // positions read and written by a launch
+    if ((persistent || (cluster_ok && ls.cl_ok)) && !P->compute_residuals && !dc.nobs) {
+      // fixed iteration count: the projectGS loop of the layer in one launch
+      CHECK(fixed_loop(sweep_bytes_of(bytes_per_tet()), 0.0, [&](int n) -> int {
+        return persistent ? launch_persistent(ls, dint, L, cd, P, n, bodyWork, w)
+                          : launch_cluster(ls, dint, L, cd, P, n, bodyWork, w);
+      }));
       if (ls.nb > 0) {
         k_finish_layer<R><<<ls.n_items, kBodyThreads, 0, stream>>>(L, w.bodies.as<Body>(), p, resv, ri, rigidLayer ? 1 : 0);
         CU(cudaGetLastError());
@@ -2825,23 +2840,9 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
         (!flow_layer(ls) || (dc.nobs > 0 && !dc.colored))) {
       // a body-free layer with a fixed iteration count: one launch, a CTA per
       // group of components
-      const int iters = std::max(ld->iterations[layer], 0);
-      if (iters > 0) {
-        const bool timed = sweep_timing && tev_used + 2 <= tev.size();
-        if (timed) CHECK(record_event(tev[tev_used], capturing));
-        const HostContactGroups hcg{cd, L.ec_off, L.ec_ids, L.ec_vert, L.n_ec_groups};
-        CHECK(launch_groups(ls, dint, P, iters, dc, nK > 0 ? &hcg : nullptr));
-        if (timed) {
-          double b = 0;
-          for (int c = 0; c < C; ++c) b += ls.color_count[c] * (group_bytes_per_tet() + (ls.identity_list ? 0.0 : 4.0));
-          CHECK(record_event(tev[tev_used + 1], capturing));
-          tev_bytes[tev_used / 2] = b * iters + 2.0 * (double)N * sizeof(R4<R>);
-          tev_launches[tev_used / 2] = 1;
-          tev_used += 2;
-        }
-        ++st.launches;
-        st.totalIterations += iters;
-      }
+      const HostContactGroups hcg{cd, L.ec_off, L.ec_ids, L.ec_vert, L.n_ec_groups};
+      CHECK(fixed_loop(sweep_bytes_of(group_bytes_per_tet()), records_once,
+                       [&](int n) -> int { return launch_groups(ls, dint, P, n, dc, nK > 0 ? &hcg : nullptr); }));
       continue;
     }
     // the sweep as one launch (flow.cuh): without bodies it also takes the
@@ -2849,7 +2850,6 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
     const bool flowDev = dc.nobs > 0 && (ls.nb == 0 || dc.colored);  // contacts inside the sweep
     const bool flow = flow_layer(ls) && (!flowDev || (!ls.fl_loose_free && (!dc.colored || ls.fl_coloured)));
     const int flowAfter = !flowDev ? 0 : (dc.colored ? 2 : 1);
-    const int iters = std::max(ld->iterations[layer], 0);
     // (a loop whose stop rules run on the host synchronises after every
     // iteration, where a cooperative launch costs more than the sweep saves:
     // 393 k tets with the PCG to residual 1e-4, 56.6 ms with the colour
@@ -2859,26 +2859,15 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
     // nothing but the sweep, its contacts and the pins
     const bool flowAll = ls.nb == 0 && nK == 0 && (flow || (sweep && !dc.nobs));
     if (flowAll && !P->compute_residuals) {
-      if (iters > 0) {
-        const bool timed = sweep_timing && tev_used + 2 <= tev.size();
-        if (timed) CHECK(record_event(tev[tev_used], capturing));
-        CHECK(flow ? launch_flow(ls, dint, P, iters, true, dc, flowAfter) : launch_sweep(ls, dint, hR, iters, true));
-        if (timed) {
-          double b = 0;
-          for (int c = 0; c < C; ++c) b += ls.color_count[c] * (group_bytes_per_tet() + (ls.identity_list ? 0.0 : 4.0));
-          CHECK(record_event(tev[tev_used + 1], capturing));
-          tev_bytes[tev_used / 2] = b * iters + 2.0 * (double)N * sizeof(R4<R>);
-          tev_launches[tev_used / 2] = 1;
-          tev_used += 2;
-        }
-        ++st.launches;
-        st.totalIterations += iters;
+      CHECK(fixed_loop(sweep_bytes_of(group_bytes_per_tet()), records_once, [&](int n) -> int {
+        CHECK(flow ? launch_flow(ls, dint, P, n, true, dc, flowAfter) : launch_sweep(ls, dint, hR, n, true));
         if (np && ls.loose_pins) {
           k_pin<R><<<blocks_for((long long)np, 256), 256, 0, stream>>>(p, d_pin_dofs.as<int>(), d_pinx.as<R>(), (int)np);
           CU(cudaGetLastError());
           ++st.launches;
         }
-      }
+        return MLX_OK;
+      }));
       continue;
     }
     cudaGraphConditionalHandle h_while_cur = 0;
