@@ -298,7 +298,8 @@ int mlx_sim_set_obstacles(mlx_solver* solver, const mlx_obstacle* obstacles, int
  * `capacity` entries copied, *len = full length), the projectGS iterations of
  * all layers, runUntilResSmallerThan after the step (it carries over to the
  * next step as in xpbdLayer3D.integrate) and a status (0 ok, 1 a layer hit
- * the iteration cap of 1e6, 2 the residual array overflowed).  In a graph
+ * the iteration cap of 1e6, 2 the residual array overflowed, 3 a sweep's wait
+ * ran out).  In a graph
  * step (use_graph) the stop rules of simpleMonitorError run on the device
  * (conditional graph nodes); without a graph they run on the host. */
 int mlx_sim_monitor(mlx_solver* solver, double* residuals, int32_t capacity, int32_t* len,
@@ -341,6 +342,12 @@ int mlx_layer_pcg(mlx_solver* solver, int32_t pcg_iterations, int32_t every);
  * limit_ns (clamped to [1 ms, 2 s]) and *timed_out is set to 1.  Shows that a
  * wait that runs out ends with a status and leaves the context usable. */
 int mlx_wait_probe(int32_t device, int32_t kind, int64_t limit_ns, int32_t* timed_out);
+/* The same for the one-launch sweeps: the solver's next mlx_layer_solve or
+ * mlx_sim_step runs as if a sweep's wait for a vertex had run out before it.
+ * Such a call ends with MLX_ERR_LIMIT -- a solve with residual monitoring
+ * after the iteration that found it, whatever its stop rules -- and the calls
+ * after it are not affected. */
+int mlx_sweep_wait_probe(mlx_solver* solver);
 
 /* xpbdLayer3D.buildLayers (3d/integrator/xpbdLayer3D.m:601-619) followed by
  * xpbdLayer2D.findBoundaryVertices (2d/integrator/xpbdLayer2D.m:551-569) on

@@ -7,7 +7,9 @@
 // the step graph and each layer sits in a conditional IF node; single-thread
 // kernels apply the same rules to a state kept in device memory and set the
 // nodes' conditions (cudaGraphSetConditional).  The number of iterations of
-// a layer is capped (MonState.error = 1 and the loop ends).
+// a layer is capped (MonState.error = 1 and the loop ends), and so does a
+// sweep that gave up a wait end it (error = 3): the sweeps after it give up at
+// once, so the residual may never reach its target.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -36,7 +38,7 @@ struct MonState {
   int end_layer;
   long long it;
   int total_iterations;
-  int error;            // 1: iteration cap, 2: residualArray full
+  int error;            // 1: iteration cap, 2: residualArray full, 3: a sweep's wait ran out
   double ra[kMonCapacity];
 };
 
@@ -71,10 +73,11 @@ __global__ void k_mon_loop_begin(MonState* ms, cudaGraphConditionalHandle loop, 
 // simpleMonitorError's rules (xpbdLayer3D.m:515-544), then the loop test.
 // With ns_every > 0 it also sets `ns`, the condition of the Newton-PCG
 // correction (pcg.cuh) that closes the iteration: after every ns_every
-// iterations of the last layer, when the loop goes on.
+// iterations of the last layer, when the loop goes on.  `sweep_error`: set by
+// a sweep whose wait ran out.
 __device__ __forceinline__ void mon_iter_end(MonState* ms, cudaGraphConditionalHandle loop, int iterations,
-                                             int is_last, const MonParams& mp, cudaGraphConditionalHandle ns = 0,
-                                             int ns_every = 0) {
+                                             int is_last, const MonParams& mp, const int* sweep_error,
+                                             cudaGraphConditionalHandle ns = 0, int ns_every = 0) {
   ms->it += 1;
   ms->total_iterations += 1;
   const double newRes = ms->res;
@@ -103,6 +106,10 @@ __device__ __forceinline__ void mon_iter_end(MonState* ms, cudaGraphConditionalH
     ms->error = 1;
     ms->end_layer = 1;
   }
+  if (__ldcg(sweep_error) != 0) {
+    ms->error = 3;
+    ms->stop = 1;
+  }
   const bool go = !(ms->end_layer || ms->stop) &&
                   (ms->it <= iterations || (!ms->stop && ms->run_until >= 0 && is_last));
   cudaGraphSetConditional(loop, go ? 1u : 0u);
@@ -110,8 +117,8 @@ __device__ __forceinline__ void mon_iter_end(MonState* ms, cudaGraphConditionalH
 }
 
 __global__ void k_mon_iter_end(MonState* ms, cudaGraphConditionalHandle loop, int iterations, int is_last,
-                               MonParams mp, cudaGraphConditionalHandle ns, int ns_every) {
-  mon_iter_end(ms, loop, iterations, is_last, mp, ns, ns_every);
+                               MonParams mp, const int* sweep_error, cudaGraphConditionalHandle ns, int ns_every) {
+  mon_iter_end(ms, loop, iterations, is_last, mp, sweep_error, ns, ns_every);
 }
 
 }  // namespace mlx

@@ -709,6 +709,13 @@ struct Solver final : SolverBase {
                      const mlx_solve_params* P, int iterations, bool body_work, LayerWork& w);
   int reset_gsync();
   int check_gsync();
+  int* sweep_error() const { return reinterpret_cast<int*>(d_gsync.as<unsigned int>() + 4); }
+  int begin_sweeps();
+  int sweep_wait_probe() override {
+    probe_sweep_wait = true;
+    return MLX_OK;
+  }
+  bool probe_sweep_wait = false;  // the next call starts as if a sweep's wait had run out
   cudaLaunchConfig_t pdl_config(int grid, int block) const {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
@@ -1802,7 +1809,7 @@ int Solver<R>::launch_sweep(const LayerStatic& ls, const int* dint, R h, int ite
   a.minv = sw_minv.as<R4<R>>();
   a.rec = sw_rec.as<SweepRec<R>>();
   a.state = sw_state.as<SweepState>();
-  a.error = reinterpret_cast<int*>(d_gsync.as<unsigned int>() + 4);
+  a.error = sweep_error();
   a.pin_at = fl_pin_at.as<int>();
   a.pin_vals = d_pinx.as<R>();
   a.n_chunks = ls.sw_chunks;
@@ -1978,7 +1985,7 @@ int Solver<R>::launch_flow(const LayerStatic& ls, const int* dint, const mlx_sol
   a.lambda = fl_lam.as<R>();
   a.pin_at = fl_pin_at.as<int>();
   a.pin_vals = d_pinx.as<R>();
-  a.error = reinterpret_cast<int*>(d_gsync.as<unsigned int>() + 4);
+  a.error = sweep_error();
   a.cs = fl_cs;
   a.slots = fl_slots;
   a.iterations = iterations;
@@ -2453,6 +2460,8 @@ int Solver<R>::residual(const ContactData& cd, double contact_resistance, double
   k_finish_norm<256><<<1, 256, 0, stream>>>(partials, tetBlocks + cBlocks + dBlocks, d_scalar.as<double>());
   CU(cudaGetLastError());
   CU(cudaMemcpyAsync(h_scalar.p, d_scalar.p, sizeof(double), cudaMemcpyDeviceToHost, stream));
+  if (flow_on || sweep_on)
+    CU(cudaMemcpyAsync(h_gsync.p, d_gsync.p, sizeof(unsigned int) * 8, cudaMemcpyDeviceToHost, stream));
   CU(cudaStreamSynchronize(stream));
   *out = h_scalar.as<double>()[0];
   return MLX_OK;
@@ -2566,7 +2575,8 @@ __global__ void __launch_bounds__(256) k_residual_monitor(TetData<R> td, const R
                                                           R inv_h, double inv_h2_d, double* __restrict__ partials,
                                                           unsigned* __restrict__ ticket, MonState* ms,
                                                           cudaGraphConditionalHandle loop, int iterations, int is_last,
-                                                          MonParams mp, cudaGraphConditionalHandle ns, int ns_every) {
+                                                          MonParams mp, const int* sweep_error,
+                                                          cudaGraphConditionalHandle ns, int ns_every) {
   pdl_launch_dependents();
   pdl_wait();
   double acc[1] = {residual_tets<R, MAT>(td, pos, inv_h2, inv_h, inv_h2_d, blockIdx.x * blockDim.x + threadIdx.x,
@@ -2587,7 +2597,7 @@ __global__ void __launch_bounds__(256) k_residual_monitor(TetData<R> td, const R
   if (threadIdx.x == 0) {
     ms->res = sqrt(sum[0]);
     *ticket = 0;
-    mon_iter_end(ms, loop, iterations, is_last, mp, ns, ns_every);
+    mon_iter_end(ms, loop, iterations, is_last, mp, sweep_error, ns, ns_every);
   }
 }
 
@@ -2961,18 +2971,19 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
         cfg.numAttrs = pdl ? 1 : 0;
         const R4<R>* pc = pos();
         const double ihd = 1.0 / (h * h);
+        const int* serr = sweep_error();
         switch (mat_kind) {
           case MAT_NH:
             CU(cudaLaunchKernelEx(&cfg, k_residual_monitor<R, MAT_NH>, td, pc, ih2, ih, ihd, parts, ticket, ms, h_while_cur,
-                                  its, il, mp, h_ns, nsEvery));
+                                  its, il, mp, serr, h_ns, nsEvery));
             break;
           case MAT_STVK_BLOCKS:
             CU(cudaLaunchKernelEx(&cfg, k_residual_monitor<R, MAT_STVK_BLOCKS>, td, pc, ih2, ih, ihd, parts, ticket, ms,
-                                  h_while_cur, its, il, mp, h_ns, nsEvery));
+                                  h_while_cur, its, il, mp, serr, h_ns, nsEvery));
             break;
           default:
             CU(cudaLaunchKernelEx(&cfg, k_residual_monitor<R, MAT_STVK_LAME>, td, pc, ih2, ih, ihd, parts, ticket, ms,
-                                  h_while_cur, its, il, mp, h_ns, nsEvery));
+                                  h_while_cur, its, il, mp, serr, h_ns, nsEvery));
         }
         ++st.launches;
         CHECK(close_body());
@@ -2981,7 +2992,7 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
       if (devmon) {
         CHECK(residual_dev(&mon()->res, dc));
         if (dc.nobs) ++st.launches;
-        k_mon_iter_end<<<1, 1, 0, stream>>>(mon(), h_while_cur, ld->iterations[layer], isLast ? 1 : 0, mp, h_ns,
+        k_mon_iter_end<<<1, 1, 0, stream>>>(mon(), h_while_cur, ld->iterations[layer], isLast ? 1 : 0, mp, sweep_error(), h_ns,
                                             nsEvery);
         CU(cudaGetLastError());
         st.launches += 3;
@@ -2993,6 +3004,7 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
         auto t0 = std::chrono::steady_clock::now();
         double newRes = 0;
         CHECK(residual(cd, P->contact_resistance, h, &newRes, &dc));
+        if (flow || sweep) CHECK(check_gsync());  // (the sweeps after one that gave up do nothing)
         st.launches += dc.nobs ? 3 : 2;
         std::vector<double>& ra = st.residualArray;
         ra.push_back(newRes);
@@ -3123,17 +3135,23 @@ int Solver<R>::reset_gsync() {
   return MLX_OK;
 }
 
+// At the start of a call: the flag of a sweep that gave up is the call's own,
+// whatever the one before it ended with.
+template <typename R>
+int Solver<R>::begin_sweeps() {
+  CU(cudaMemsetAsync(sweep_error(), probe_sweep_wait ? 1 : 0, sizeof(int), stream));
+  probe_sweep_wait = false;
+  return MLX_OK;
+}
+
 // Copies the barrier error flag to the host (stream-ordered); check_gsync
 // reads it after the stream has been synchronised.
 template <typename R>
 int Solver<R>::check_gsync() {
   if (h_gsync.as<int>()[2] != 0)
     return set_error(MLX_ERR_LIMIT, "a grid barrier of the persistent layer kernel waited more than 1 s");
-  if (h_gsync.as<int>()[4] != 0) {
-    // (kept across the steps of a call; cleared once reported)
-    CU(cudaMemsetAsync(d_gsync.as<unsigned int>() + 4, 0, sizeof(int), stream));
+  if (h_gsync.as<int>()[4] != 0)  // (kept across the steps of a call)
     return set_error(MLX_ERR_LIMIT, "a tet of a sweep waited more than 1 s for a vertex");
-  }
   return MLX_OK;
 }
 
@@ -3440,6 +3458,7 @@ int Solver<R>::layer_solve(const mlx_layer_desc* ld, const mlx_solve_params* P, 
   st.runUntil = P->run_until;
   st.sumNonMon = in->sum_non_monitored_time;
   CHECK(reset_gsync());
+  CHECK(begin_sweeps());
   // A call of the same shape as the previous one replays it as a graph; with
   // residual monitoring the stop rules then run on the device (monitor.cuh:
   // the same rules and residual bits as the host loop), the residual array
@@ -4610,6 +4629,7 @@ int Solver<R>::sim_step(int nsteps, int use_graph, double* device_ms) {
   if (!sim.ready) return set_error(MLX_ERR_ARGUMENT, "sim_setup has not been called");
   if (nsteps < 0) return set_error(MLX_ERR_ARGUMENT, "nsteps < 0");
   DeviceGuard g(device);
+  CHECK(begin_sweeps());
   if (use_graph && !sim.graph) {
     cudaGraph_t graph = nullptr;
     CU(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
@@ -4661,7 +4681,7 @@ int Solver<R>::sim_step(int nsteps, int use_graph, double* device_ms) {
     cudaEventDestroy(e1);
   }
   CU(cudaStreamSynchronize(stream));
-  CHECK(check_gsync());
+  if (nsteps > 0) CHECK(check_gsync());
   return MLX_OK;
 }
 
@@ -4937,6 +4957,12 @@ int mlx_pcg_solve(mlx_solver* s, double h, const double* b, int32_t iterations, 
   return mlx::guarded([&]() -> int {
     if (!s) return set_error(MLX_ERR_ARGUMENT, "null solver");
     return s->impl->pcg_solve(h, b, iterations, x, resvec);
+  });
+}
+int mlx_sweep_wait_probe(mlx_solver* s) {
+  return mlx::guarded([&]() -> int {
+    if (!s) return set_error(MLX_ERR_ARGUMENT, "null solver");
+    return s->impl->sweep_wait_probe();
   });
 }
 int mlx_sim_contact_count(mlx_solver* s, int32_t* n) {
