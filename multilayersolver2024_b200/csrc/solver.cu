@@ -19,6 +19,7 @@
 #include "groups.cuh"
 #include "flow.cuh"
 #include "sweep.cuh"
+#include "sweep_times.h"
 #include "layers_dev.cuh"
 #include "contacts.cuh"
 #include "monitor.cuh"
@@ -339,6 +340,7 @@ struct LayerStatic {
   bool identity_list = false;
   std::vector<int> color_count;  // per colour: number of elastic tets
   std::vector<int> color_start;  // per colour: start in the elastic list
+  int tets = 0, colours = 0;     // elastic tets, colours with any
   std::vector<int> packed;       // body_vert_off | body_verts | bnd_off | bnd_verts | list | vert_body
   size_t o_bvo = 0, o_bv = 0, o_bo = 0, o_bnd = 0, o_list = 0, o_vb = 0, o_cstart = 0, o_ccount = 0;
   int n_bnd = 0;
@@ -678,7 +680,22 @@ struct Solver final : SolverBase {
   bool fl_iso = false;                     // undamped blocks stored as MAT_STVK_ISO
   DevBuf fl_lam;
   int flow_mat() const { return fl_iso ? (int)MAT_STVK_ISO : mat_kind; }
-  bool flow_forced = false;  // MLXPBD_FLOW=1: no other path beside it
+  bool flow_forced = false;  // MLXPBD_FLOW=1 or 2: no other path beside it
+  SweepMat sweep_mat() const {
+    return mat_kind == MAT_NH ? SWEEP_NH
+           : mat_kind == MAT_STVK_BLOCKS ? (damp ? SWEEP_BLOCKS_DAMPED : SWEEP_BLOCKS)
+                                         : (damp ? SWEEP_LAME_DAMPED : SWEEP_LAME);
+  }
+  bool flow_pays(const LayerStatic& ls, bool once, bool contacts, bool colored) const;
+  bool sweep_pays(const LayerStatic& ls) const;
+  // Coloured contacts of a body-free layer that the component groups could
+  // take.  Resting blocks, us per sweep here / there, by chunks of the largest
+  // part: FP32 StVK 20 45/54, 81 48/87, 140 118/92, 166 105/90, 875 470/302;
+  // Neo-Hookean 140 87/84, 648 252/251, 875 338/278; damped 166 131/136.  FP64
+  // is never longer here (875: 394/391).
+  bool flow_keeps_coloured(const LayerStatic& ls) const {
+    return flow_forced || sizeof(R) == 8 || ls.fl_max <= (mat_kind != MAT_NH && !(damp && mat_kind == MAT_STVK_BLOCKS) ? 110 : 700);
+  }
   int plan_flow(const mlx_mesh_desc* md);
   int upload_pin_at();
   int build_flow(LayerStatic& ls, const std::vector<int>& list);
@@ -1498,7 +1515,8 @@ static int flow_limits(int device, bool fp64, int mat, bool damp, int threads, F
 template <typename R>
 int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
   const char* env = std::getenv("MLXPBD_FLOW");
-  const bool force = flow_forced = env && std::string(env) == "1";
+  const bool force = env && std::string(env) == "1";
+  flow_forced = force || (env && std::string(env) == "2");
   if ((env && std::string(env) == "0") || persistent || cluster_ok || std::getenv("MLXPBD_PDL")) return MLX_OK;
   if (env && std::string(env) == "2") return plan_sweep();
   if (!force && std::getenv("MLXPBD_GROUPS")) return MLX_OK;
@@ -1542,6 +1560,8 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
   fl_smem = lim.smem;
   int want_cs = 0;
   if (const char* q = std::getenv("MLXPBD_FLOW_CS")) want_cs = std::atoi(q);
+  const bool fp64 = sizeof(R) == 8;
+  const SweepTimes& times = sweep_times(fp64, sweep_mat());
   struct Plan {
     std::vector<int> first;  // [G cs + 1] first position of every part in the element order
     int G = 0, cs = 0, slots = 0;
@@ -1601,13 +1621,7 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
       c = e;
     }
     pl.first.push_back(T);
-    // Measured (B200, Neo-Hookean FP32, us per sweep): 0.9 per colour while the
-    // warps wait for records, 0.13 per chunk of the largest part while they
-    // share the SM, and both add up like independent parts (27,648 tets on
-    // 16 / 8 CTAs: 29 / 34; 10,368 on 4 / 2 / 1: 30 / 35 / 46; 98,304 on 16: 41;
-    // 393,216 on 16: 112).
-    const double chain = 0.9 * C, issue = 0.13 * ((double)pl.most / 32.0 + 0.5 * C);
-    pl.t = std::sqrt(chain * chain + issue * issue);
+    pl.t = flow_us(times, fp64, sweep_mat(), C, (double)pl.most / 32.0 + 0.5 * C, pl.G, cs, false, false);
     plans.push_back(pl);
   }
   // the shortest estimate whose slots and chunk barriers (every colour rounds
@@ -1615,10 +1629,14 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
   std::stable_sort(plans.begin(), plans.end(), [](const Plan& x, const Plan& y) { return x.t < y.t; });
   for (size_t i = 0; i + 1 < plans.size(); ++i)
     if (plans[i + 1].cs < plans[i].cs && plans[i + 1].t * 0.97 < plans[i].t) std::swap(plans[i], plans[i + 1]);
-  // (none of them is tried when the sweep through L2 is estimated shorter)
-  const double t_l2 = 1.55 * C + 3.3e-5 * (double)T;
+  // (none of them is tried when another path is estimated shorter: the sweep
+  // through L2, or the colour launches, whose recorded chain of dependents
+  // takes longer in a fixed loop than one by one)
+  const double t_colours = 1.05 * colours_us(times, C, T);
+  const double t_l2 = fp64 ? 1e30 : l2_us(times, C, T, false);
+  const double t_other = std::min(t_l2, t_colours);
   for (Plan& pl : plans) {
-    if (!force && pl.t > t_l2) break;
+    if (!force && pl.t > t_other) break;
     const long long bars = pl.most / 32 + C;
     if (bars > kFlowMaxChunks) continue;
     count(pl, eslot);
@@ -1626,10 +1644,7 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
     best = pl;
     break;
   }
-  // A launch per colour takes ~1.75 us plus its tets' traffic (58 us per sweep
-  // of 98 k tets, 85 of 393 k), the sweep through L2 less than that at any
-  // size (53 and 62 us).
-  if (best.t < 0) return force ? MLX_OK : plan_sweep();
+  if (best.t < 0) return force || t_l2 > t_colours ? MLX_OK : plan_sweep();
   if (best.cs > 1 && best.sum > 3 * (long long)N / 2) {
     // parts that share many vertices (an element order of thin slabs): cut
     // the breadth-first order instead where that shares fewer
@@ -1915,6 +1930,30 @@ int Solver<R>::build_flow(LayerStatic& ls, const std::vector<int>& clist) {
   }
   ls.fl_ok = true;
   return MLX_OK;
+}
+
+// Whether the dataflow sweep is estimated shorter than a layer's colour
+// launches (sweep_times.h).  once: one iteration per launch.  Contacts add a
+// launch to the colour launches (5 us), or lengthen them all (10 us and 17 per
+// 100,000 vertices that may be in contact).
+template <typename R>
+bool Solver<R>::flow_pays(const LayerStatic& ls, bool once, bool contacts, bool colored) const {
+  if (flow_forced || (!once && !contacts)) return true;
+  const SweepTimes& t = sweep_times(sizeof(R) == 8, sweep_mat());
+  const double by_colour = colours_us(t, colored ? C : ls.colours, ls.tets);
+  return flow_us(t, sizeof(R) == 8, sweep_mat(), ls.colours, ls.fl_max, fl_G, fl_cs, once, contacts) <=
+         by_colour + (colored ? 10.0 + 1.7e-4 * N : contacts ? 5.0 : 0.0);
+}
+
+// Whether one sweep through L2 is estimated a tenth shorter than a layer's
+// colour launches (a cooperative launch does not overlap the kernel before
+// it).  FP32 only.
+template <typename R>
+bool Solver<R>::sweep_pays(const LayerStatic& ls) const {
+  if (flow_forced) return true;
+  if (sizeof(R) == 8) return false;
+  const SweepTimes& t = sweep_times(false, sweep_mat());
+  return 1.1 * l2_us(t, ls.colours, ls.tets, true) <= colours_us(t, ls.colours, ls.tets);
 }
 
 // Fills the layer's chunk planes and counts, once its packed lists are on the
@@ -2219,6 +2258,8 @@ int Solver<R>::build_static(const mlx_layer_desc* ld, int col, LayerStatic& ls, 
       if (isE[s2e[s]]) list.push_back(s);
     ls.color_count[c] = (int)list.size() - ls.color_start[c];
   }
+  ls.tets = (int)list.size();
+  ls.colours = (int)std::count_if(ls.color_count.begin(), ls.color_count.end(), [](int n) { return n > 0; });
   ls.identity_list = (int)list.size() == T;
   // bodies
   std::vector<int> bvo(nb + 1, 0), bo(nb + 1, 0);
@@ -2847,7 +2888,7 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
       continue;
     }
     if (groups_ok && ls.gr_ok && ls.nb == 0 && !P->compute_residuals && (gr_cs == 1 || (!dc.nobs && nK == 0)) &&
-        (!flow_layer(ls) || (dc.nobs > 0 && !dc.colored))) {
+        (!flow_layer(ls) || (dc.nobs > 0 && (!dc.colored || !flow_keeps_coloured(ls))))) {
       // a body-free layer with a fixed iteration count: one launch, a CTA per
       // group of components
       const HostContactGroups hcg{cd, L.ec_off, L.ec_ids, L.ec_vert, L.n_ec_groups};
@@ -2858,14 +2899,20 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
     // the sweep as one launch (flow.cuh): without bodies it also takes the
     // device-detected contacts and the pins, and a fixed number of iterations
     const bool flowDev = dc.nobs > 0 && (ls.nb == 0 || dc.colored);  // contacts inside the sweep
-    const bool flow = flow_layer(ls) && (!flowDev || (!ls.fl_loose_free && (!dc.colored || ls.fl_coloured)));
+    // a fixed loop in one launch, or one iteration per launch
+    const bool once = P->compute_residuals || ls.nb > 0 || nK > 0;
+    const bool flow = flow_layer(ls) && (!flowDev || (!ls.fl_loose_free && (!dc.colored || ls.fl_coloured))) &&
+                      flow_pays(ls, once, flowDev, dc.colored);
     const int flowAfter = !flowDev ? 0 : (dc.colored ? 2 : 1);
     // (a loop whose stop rules run on the host synchronises after every
     // iteration, where a cooperative launch costs more than the sweep saves:
     // 393 k tets with the PCG to residual 1e-4, 56.6 ms with the colour
-    // launches and 66.4 with it)
+    // launches and 66.4 with it.  FP32 results are the same bits; in FP64, where
+    // the two kernels differ in their fused multiply-adds, the sweep runs only
+    // when asked for, then under either kind of rules)
     const bool hostRules = P->compute_residuals && !devmon;
-    const bool sweep = !dc.colored && !hostRules && sweep_layer(ls, P->compute_residuals ? 1 : iters);
+    const bool sweep = !dc.colored && sweep_layer(ls, once ? 1 : iters) &&
+                       (flow_forced || (!once && !dc.nobs) || (!hostRules && sweep_pays(ls)));
     // nothing but the sweep, its contacts and the pins
     const bool flowAll = ls.nb == 0 && nK == 0 && (flow || (sweep && !dc.nobs));
     if (flowAll && !P->compute_residuals) {
