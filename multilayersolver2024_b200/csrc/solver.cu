@@ -756,6 +756,7 @@ struct Solver final : SolverBase {
   long long sweep_launches = 0;
   double bytes_per_tet() const;
   double group_bytes_per_tet() const;
+  double flow_bytes_per_tet() const;
   int record_event(cudaEvent_t e, bool capturing);
   int enable_sweep_timing(int on) override;
   int sweep_stats(double* ms, double* bytes, long long* launches, int reset) override;
@@ -793,11 +794,12 @@ struct Solver final : SolverBase {
     }
     if (sweep_on && t.empty())
       return "version-ordered sweeps, one launch each on " + std::to_string(sw_sms) +
-             " CTAs; contacts coloured with the elastic constraints: one launch per colour";
+             " CTAs; one launch per colour where that is shorter and with coloured contacts";
     if (flow_on && t.empty())
       return "dataflow sweeps, one launch each: " + std::to_string(fl_G) + " clusters of " + std::to_string(fl_cs) +
-             " CTAs each owning whole components (records in shared memory); layers they do not cover: one launch per "
-             "colour (programmatic dependent launches)";
+             " CTAs each owning whole components (records in shared memory); " +
+             (groups_ok ? std::to_string(gr_G) + " component groups for contacts of body-free layers; " : std::string()) +
+             "one launch per colour where that is shorter";
     return std::string("one launch per colour") + (pdl ? " (programmatic dependent launches)" : "") + t;
   }
   long long launches_last_call() const override { return last_launches; }
@@ -2868,10 +2870,8 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
       }
       return MLX_OK;
     };
-    auto sweep_bytes_of = [&](double per_tet) {
-      double b = 0;
-      for (int c = 0; c < C; ++c) b += ls.color_count[c] * (per_tet + (ls.identity_list ? 0.0 : 4.0));
-      return b;
+    auto sweep_bytes_of = [&](double per_tet, bool list = true) {  // (the dataflow path's planes need no list)
+      return ls.tets * (per_tet + (list && !ls.identity_list ? 4.0 : 0.0));
     };
     const double records_once = 2.0 * (double)N * sizeof(R4<R>);  // positions read and written by a launch
     if ((persistent || (cluster_ok && ls.cl_ok)) && !P->compute_residuals && !dc.nobs) {
@@ -2916,7 +2916,8 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
     // nothing but the sweep, its contacts and the pins
     const bool flowAll = ls.nb == 0 && nK == 0 && (flow || (sweep && !dc.nobs));
     if (flowAll && !P->compute_residuals) {
-      CHECK(fixed_loop(sweep_bytes_of(group_bytes_per_tet()), records_once, [&](int n) -> int {
+      CHECK(fixed_loop(sweep_bytes_of(flow ? flow_bytes_per_tet() : bytes_per_tet(), !flow), flow ? records_once : 0.0,
+                       [&](int n) -> int {
         CHECK(flow ? launch_flow(ls, dint, P, n, true, dc, flowAfter) : launch_sweep(ls, dint, hR, n, true));
         if (np && ls.loose_pins) {
           k_pin<R><<<blocks_for((long long)np, 256), 256, 0, stream>>>(p, d_pin_dofs.as<int>(), d_pinx.as<R>(), (int)np);
@@ -2953,7 +2954,7 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
         CHECK(flow ? launch_flow(ls, dint, P, 1, flowAll, dc, flowAfter) : launch_sweep(ls, dint, hR, 1, flowAll));
         ++st.launches;
         sweep_l = 1;
-        for (int c = 0; c < C; ++c) sweep_b += ls.color_count[c] * (bytes_per_tet() + (ls.identity_list ? 0.0 : 4.0));
+        sweep_b = flow ? sweep_bytes_of(flow_bytes_per_tet(), false) + records_once : sweep_bytes_of(bytes_per_tet());
       }
       for (int c = 0; c < C && !flow && !sweep; ++c) {
         if (ls.color_count[c] == 0 && !dc.colored) continue;
@@ -4558,6 +4559,17 @@ double Solver<R>::group_bytes_per_tet() const {
   const int nl = mat_kind == MAT_NH ? 2 : 6;
   const double vol = mat_kind == MAT_NH ? 0 : r;
   double b = 16 + 9 * r + vol + mat_stride(mat_kind) * r + 2 * nl * r;
+  if (damp) b += 16 + 4 * 4 * r;
+  return b;
+}
+
+template <typename R>
+double Solver<R>::flow_bytes_per_tet() const {
+  // the dataflow path reads chunk planes instead (rest data in whole vectors,
+  // 32 bytes of corner words; vertex ids and four step-start records with
+  // Rayleigh damping) and the multipliers, read and written
+  const double r = sizeof(R);
+  double b = 4 * r * flow_planes_of(flow_mat()) + 32 + 2 * (mat_kind == MAT_NH ? 2 : 6) * r;
   if (damp) b += 16 + 4 * 4 * r;
   return b;
 }
