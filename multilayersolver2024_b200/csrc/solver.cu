@@ -1623,7 +1623,9 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
       c = e;
     }
     pl.first.push_back(T);
-    pl.t = flow_us(times, fp64, sweep_mat(), C, (double)pl.most / 32.0 + 0.5 * C, pl.G, cs, false, false);
+    // (compared with one another without what busy SMs cost: more CTAs were
+    // never slower, 36 blocks of 10,368 tets FP64 on 4 / 2 CTAs each 44 / 53)
+    pl.t = flow_us(times, fp64, sweep_mat(), C, (double)pl.most / 32.0 + 0.5 * C, 1, 1, false, false);
     plans.push_back(pl);
   }
   // the shortest estimate whose slots and chunk barriers (every colour rounds
@@ -1638,7 +1640,8 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
   const double t_l2 = fp64 ? 1e30 : l2_us(times, C, T, false);
   const double t_other = std::min(t_l2, t_colours);
   for (Plan& pl : plans) {
-    if (!force && pl.t > t_other) break;
+    if (!force && flow_us(times, fp64, sweep_mat(), C, (double)pl.most / 32.0 + 0.5 * C, pl.G, pl.cs, false, false) > t_other)
+      break;
     const long long bars = pl.most / 32 + C;
     if (bars > kFlowMaxChunks) continue;
     count(pl, eslot);
