@@ -211,11 +211,13 @@ static __global__ void k_scatter_zero(const int* __restrict__ list, int n, int* 
   if (i < n) at[list[i]] = 0;
 }
 // Corner words of the sweep through L2: the rank of every elastic tet at its
-// vertices; at[s] >= 0 marks the layer's tets, D receives the longest chain.
+// vertices; at[s] >= 0 marks the layer's tets, D receives the longest chain,
+// touched the vertices with any.
 static __global__ void __launch_bounds__(128) k_sweep_link(const int* __restrict__ voff, const int* __restrict__ vcor,
                                                            const int* __restrict__ at, const int* __restrict__ pin_at,
                                                            int N, unsigned short* __restrict__ corner,
-                                                           int* __restrict__ loose, int* __restrict__ D) {
+                                                           int* __restrict__ loose, int* __restrict__ D,
+                                                           int* __restrict__ touched) {
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= N) return;
   const bool pin = pin_at && (pin_at[3 * v] >= 0 || pin_at[3 * v + 1] >= 0 || pin_at[3 * v + 2] >= 0);
@@ -229,6 +231,7 @@ static __global__ void __launch_bounds__(128) k_sweep_link(const int* __restrict
   if (last >= 0) corner[last] |= kSweepLast;
   else if (pin) *loose = 1;
   atomicMax(D, n);
+  if (n > 0) atomicAdd(touched, 1);
 }
 template <typename R>
 __global__ void k_corner_masses(const int4* __restrict__ vid, const double* __restrict__ mass3, int T,
@@ -363,7 +366,7 @@ struct LayerStatic {
   size_t o_fcorner = 0, o_fvid = 0;
   // sweeps through L2 (sweep.cuh): chunks and corner words
   bool sw_ok = false;
-  int sw_chunks = 0, sw_D = 0;
+  int sw_chunks = 0, sw_D = 0, sw_vertices = 1;  // longest chain, vertices with any
   size_t o_swch = 0;
   DevBuf sw_corner;
   // cluster kernel: (colour, part) ranges of the elastic tets, colours with work
@@ -1625,7 +1628,7 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
     pl.first.push_back(T);
     // (compared with one another without what busy SMs cost: more CTAs were
     // never slower, 36 blocks of 10,368 tets FP64 on 4 / 2 CTAs each 44 / 53)
-    pl.t = flow_us(times, fp64, sweep_mat(), C, (double)pl.most / 32.0 + 0.5 * C, 1, 1, false, false);
+    pl.t = flow_us(times, fp64, sweep_mat(), C, (double)pl.most / 32.0 + 0.5 * C, 1, false, false);
     plans.push_back(pl);
   }
   // the shortest estimate whose slots and chunk barriers (every colour rounds
@@ -1637,10 +1640,10 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
   // through L2, or the colour launches, whose recorded chain of dependents
   // takes longer in a fixed loop than one by one)
   const double t_colours = 1.05 * colours_us(times, C, T);
-  const double t_l2 = fp64 ? 1e30 : l2_us(times, C, T, false);
+  const double t_l2 = fp64 ? 1e30 : l2_us(times, C * 2.0 / 3.0, T, false);
   const double t_other = std::min(t_l2, t_colours);
   for (Plan& pl : plans) {
-    if (!force && flow_us(times, fp64, sweep_mat(), C, (double)pl.most / 32.0 + 0.5 * C, pl.G, pl.cs, false, false) > t_other)
+    if (!force && flow_us(times, fp64, sweep_mat(), C, (double)pl.most / 32.0 + 0.5 * C, pl.G * pl.cs, false, false) > t_other)
       break;
     const long long bars = pl.most / 32 + C;
     if (bars > kFlowMaxChunks) continue;
@@ -1809,13 +1812,14 @@ int Solver<R>::link_sweep(LayerStatic& ls) {
   for (int c = 0; c < C; ++c) n += ls.color_count[c];
   if (list && n > 0) k_scatter_zero<<<blocks_for(n, 256), 256, 0, stream>>>(list, n, at);
   k_sweep_link<<<blocks_for(N, 128), 128, 0, stream>>>(ch_off.as<int>(), ch_cor.as<int>(), at, fl_pin_at.as<int>(), N,
-                                                       ls.sw_corner.template as<unsigned short>(), at + T, at + T + 1);
+                                                       ls.sw_corner.template as<unsigned short>(), at + T, at + T + 1, at + T + 2);
   CU(cudaGetLastError());
   int* hs = h_scalar.as<int>();
-  CU(cudaMemcpyAsync(hs, at + T, sizeof(int) * 2, cudaMemcpyDeviceToHost, stream));
+  CU(cudaMemcpyAsync(hs, at + T, sizeof(int) * 3, cudaMemcpyDeviceToHost, stream));
   CU(cudaStreamSynchronize(stream));
   ls.loose_pins = hs[0] != 0;
   ls.sw_D = std::max(hs[1], 1);
+  ls.sw_vertices = std::max(hs[2], 1);
   return MLX_OK;
 }
 
@@ -1946,7 +1950,7 @@ bool Solver<R>::flow_pays(const LayerStatic& ls, bool once, bool contacts, bool 
   if (flow_forced || (!once && !contacts)) return true;
   const SweepTimes& t = sweep_times(sizeof(R) == 8, sweep_mat());
   const double by_colour = colours_us(t, colored ? C : ls.colours, ls.tets);
-  return flow_us(t, sizeof(R) == 8, sweep_mat(), ls.colours, ls.fl_max, fl_G, fl_cs, once, contacts) <=
+  return flow_us(t, sizeof(R) == 8, sweep_mat(), ls.colours, ls.fl_max, fl_G * fl_cs, once, contacts) <=
          by_colour + (colored ? 10.0 + 1.7e-4 * N : contacts ? 5.0 : 0.0);
 }
 
@@ -1958,7 +1962,7 @@ bool Solver<R>::sweep_pays(const LayerStatic& ls) const {
   if (flow_forced) return true;
   if (sizeof(R) == 8) return false;
   const SweepTimes& t = sweep_times(false, sweep_mat());
-  return 1.1 * l2_us(t, ls.colours, ls.tets, true) <= colours_us(t, ls.colours, ls.tets);
+  return 1.1 * l2_us(t, 4.0 * ls.tets / ls.sw_vertices, ls.tets, true) <= colours_us(t, ls.colours, ls.tets);
 }
 
 // Fills the layer's chunk planes and counts, once its packed lists are on the

@@ -19,8 +19,8 @@
 //   64 blocks of 10,368    FP32 92/100/121   FP64 123/202/166
 // The sweep through L2 loses in FP64 at every size (its records are three
 // words); above 1.3 M tets its records and rest data leave L2 and it loses in FP32.
-// Where the estimates are within a tenth of one another they can pick the
-// longer path: nine blocks of 83 k tets, coloured contacts, FP32 128 here / 117.
+// Estimates within a tenth of one another can pick the longer path: nine
+// damped FP64 blocks of 83 k tets in a fixed loop take 204 here, 186 by colours.
 #pragma once
 
 #include <algorithm>
@@ -34,35 +34,34 @@ struct SweepTimes {
   double contact;  // dataflow: the same with every 3rd to 13th vertex in contact
   double colour;   // a colour launch
   double tet;      // colour launches: a tet's traffic
-  double l2;       // the sweep through L2, per colour
+  double l2;       // the sweep through L2: a tet of a vertex's chain
 };
 
 enum SweepMat : int { SWEEP_NH, SWEEP_BLOCKS, SWEEP_BLOCKS_DAMPED, SWEEP_LAME, SWEEP_LAME_DAMPED };
 
 inline const SweepTimes& sweep_times(bool fp64, SweepMat m) {
-  static const SweepTimes t[2][5] = {{{0.98, 0.137, 0.36, 1.80, 5.0e-5, 1.9},
-                                      {0.98, 0.137, 0.50, 1.92, 7.5e-5, 1.9},
-                                      {1.50, 0.21, 0.70, 2.30, 6.5e-5, 2.55},
-                                      {1.07, 0.145, 0.55, 2.27, 5.5e-5, 2.0},
-                                      {1.30, 0.17, 0.60, 2.50, 5.5e-5, 2.3}},
-                                     {{1.10, 0.215, 0.30, 2.10, 1.15e-4, 3.2},
-                                      {1.56, 0.28, 0.62, 2.65, 1.4e-4, 3.6},
-                                      {2.30, 0.43, 0.65, 3.35, 1.0e-4, 4.4},
-                                      {1.58, 0.27, 0.60, 2.90, 1.1e-4, 3.8},
-                                      {1.88, 0.34, 0.60, 3.25, 9.0e-5, 4.3}}};
+  static const SweepTimes t[2][5] = {{{0.98, 0.137, 0.36, 1.80, 5.0e-5, 2.85},
+                                      {0.98, 0.137, 0.50, 1.92, 7.5e-5, 2.85},
+                                      {1.50, 0.21, 0.70, 2.30, 6.5e-5, 3.8},
+                                      {1.07, 0.145, 0.55, 2.27, 5.5e-5, 3.0},
+                                      {1.30, 0.17, 0.60, 2.50, 5.5e-5, 3.45}},
+                                     {{1.10, 0.215, 0.30, 2.10, 1.15e-4, 4.8},
+                                      {1.56, 0.28, 0.62, 2.65, 1.4e-4, 5.4},
+                                      {2.30, 0.37, 0.65, 3.35, 1.4e-4, 6.6},
+                                      {1.58, 0.27, 0.60, 2.90, 1.1e-4, 5.7},
+                                      {1.88, 0.34, 0.60, 3.25, 9.0e-5, 6.4}}};
   return t[fp64 ? 1 : 0][m];
 }
 
 // The dataflow sweep of `colours` colours whose largest part has `chunks`
-// chunks, on `clusters` clusters of `cs` CTAs.  A chunk takes longer where
-// most SMs are busy (rest data from the shared L2), the more on clusters of 16
-// (83 k tets per cluster, FP32, 1 / 4 / 9 clusters: 40 / 45 / 69).  once: one
-// iteration per launch, which reads positions and multipliers anew (FP64, 20 /
-// 140 / 875 chunks of 148 CTAs: 18 of 50, 32 of 97, 419 of 717).
-inline double flow_us(const SweepTimes& t, bool fp64, SweepMat m, double colours, double chunks, int clusters, int cs,
-                      bool once, bool contacts) {
-  const double busy = std::min(1.0, clusters * cs / 148.0);
-  const double shared = 1.0 + std::max(0.0, busy - 0.25) * (cs >= 16 ? 2.0 : 1.1);
+// chunks, on `ctas` CTAs.  A chunk takes longer where most SMs are busy: 83 k
+// tets per 16 CTAs, 1 / 4 clusters 40 / 45 us FP32, 92 / 131 damped FP64.
+// once: one iteration per launch, which reads positions and multipliers anew
+// (FP64, 20 / 140 / 875 chunks of 148 CTAs: 18 of 50, 32 of 97, 419 of 717).
+inline double flow_us(const SweepTimes& t, bool fp64, SweepMat m, double colours, double chunks, int ctas, bool once,
+                      bool contacts) {
+  const double busy = std::min(1.0, ctas / 148.0);
+  const double shared = 1.0 + 0.9 * std::max(0.0, busy - 0.25);
   const double chain = t.chain * colours + (contacts ? 17.0 : 0.0);
   const double issue = chunks * (contacts ? t.contact * std::max(1.0, shared / 1.36) : t.chunk * shared);
   const double q = std::max(0.0, chunks - 0.5 * colours);  // (half a chunk per colour is rounding)
@@ -71,9 +70,11 @@ inline double flow_us(const SweepTimes& t, bool fp64, SweepMat m, double colours
   return std::sqrt(chain * chain + issue * issue) + (once ? again : 0.0);
 }
 inline double colours_us(const SweepTimes& t, double colours, double tets) { return t.colour * colours + t.tet * tets; }
-// The sweep through L2.
-inline double l2_us(const SweepTimes& t, double colours, double tets, bool once) {
-  return t.l2 * colours + 2e-5 * tets + 8e-5 * std::max(0.0, tets - 8.5e5) + (once ? 6.0 : 0.0);
+// The sweep through L2; chain: tets at a vertex, on average (22 of the beams'
+// 33 colours; layers with bodies 13 to 15, where it is 11 us shorter than the
+// colour launches at 120 to 220 k tets).
+inline double l2_us(const SweepTimes& t, double chain, double tets, bool once) {
+  return t.l2 * chain + 2e-5 * tets + 8e-5 * std::max(0.0, tets - 8.5e5) + (once ? 6.0 : 0.0);
 }
 
 }  // namespace mlx

@@ -26,10 +26,10 @@ def _integ(hanging):
     return integ
 
 
-def _three_calls(m, prec, layers, iterations, hanging):
+def _three_calls(m, prec, layers, iterations, hanging, material="lame"):
     case = Case(m, layers, iterations, seed=7, integ=_integ(hanging), h=1.0 / 60.0)
-    s = Solver(m, precision=prec, material="lame")
-    out = [case.product(prec, "lame", solver=s) for _ in range(3)]
+    s = Solver(m, precision=prec, material=material)
+    out = [case.product(prec, material, solver=s) for _ in range(3)]
     path = s.launch_path
     s.close()
     for xi, _, ra, ru, lam, it in out[1:]:
@@ -43,9 +43,11 @@ def _three_calls(m, prec, layers, iterations, hanging):
 @pytest.mark.parametrize("energy", [NH, STVK])
 @pytest.mark.parametrize("prec", [_lib.MLX_FP32, _lib.MLX_FP64])
 @pytest.mark.parametrize("path", ["1", "2"])
-def test_replays_of_a_forced_path(gpu, monkeypatch, energy, prec, path):
+@pytest.mark.parametrize("material,alpha1", [("lame", 0.0), ("blocks", 0.0), ("blocks", 0.01)])
+def test_replays_of_a_forced_path(gpu, monkeypatch, energy, prec, path, material, alpha1):
     monkeypatch.setenv("MLXPBD_FLOW", path)
-    _three_calls(block_mesh(dims=(8, 3, 3), energy=energy, seed=5), prec, [50, 0], [2, 3], 40)
+    m = block_mesh(dims=(9, 5, 4), energy=energy, seed=5, alpha1=alpha1)
+    _three_calls(m, prec, [50, 0], [2, 3], 40, material)
 
 
 @pytest.mark.parametrize("prec", [_lib.MLX_FP32, _lib.MLX_FP64])
