@@ -352,7 +352,7 @@ struct LayerStatic {
   // component-group path (groups.cuh): (colour, group) ranges of the elastic tets
   bool gr_ok = false;
   int gr_one = 0;
-  size_t o_goff = 0;
+  DevBuf gr_off;
   std::vector<int> tile;  // block size of each colour kernel (0 = default), set by the autotuner
   // dataflow path (flow.cuh): chunks of each part, corner words and slots
   bool fl_ok = false;
@@ -653,7 +653,11 @@ struct Solver final : SolverBase {
   size_t gr_smem = 0;
   std::vector<int> tgroup_sorted;  // group of each tet, sorted order
   DevBuf d_gv0, d_tloc, d_gpin;
-  int plan_groups(const mlx_mesh_desc* md);
+  int plan_groups();
+  bool groups_planned = false;
+  std::vector<int> comp_root;
+  void find_components(const mlx_mesh_desc* md);
+  int build_groups(LayerStatic& ls);
   // buildLayers + findBoundaryVertices on the device (layers_dev.cuh)
   DevBuf lb_p, lb_oldp, lb_dminv, lb_norms, lb_norms_sorted, lb_elems, lb_order, lb_rank, lb_forced, lb_parent,
       lb_rep, lb_root, lb_flag, lb_scan, lb_sets, lb_key, lb_touch, lb_isE, lb_isBV, lb_isRV, lb_body, lb_small,
@@ -679,7 +683,7 @@ struct Solver final : SolverBase {
   // MAT_STVK_ISO values, k_flow_link's scratch
   DevBuf fl_tables;
   DevPart fl_partd, fl_srcd, ch_off, ch_cor, fl_pin_at, fl_mat, fl_at;
-  int flow_tables();
+  int flow_tables(bool parts);
   bool fl_iso = false;                     // undamped blocks stored as MAT_STVK_ISO
   DevBuf fl_lam;
   int flow_mat() const { return fl_iso ? (int)MAT_STVK_ISO : mat_kind; }
@@ -1018,8 +1022,14 @@ int Solver<R>::create(const mlx_mesh_desc* md) {
     CU(cudaMemcpyAsync(d_pin_dofs.p, pinned.data(), sizeof(int) * pinned.size(), cudaMemcpyHostToDevice, stream));
   vid_sorted = vid;
   if (cluster_ok) vowner = mp.vowner;
+  // (beside the dataflow sweeps the groups take contacts only: planned with
+  // the first obstacles)
   CHECK(plan_flow(md));
-  if (!sweep_on && !flow_forced) CHECK(plan_groups(md));
+  if (!flow_on && !sweep_on && !flow_forced) {
+    find_components(md);
+    CHECK(plan_groups());
+  }
+  if (!flow_on || flow_forced) std::vector<int>().swap(comp_root);
   if (md->mu && md->lambda) {
     pcg_G.resize(9 * (size_t)T);
     pcg_vol.resize(T);
@@ -1169,35 +1179,20 @@ static const void* cgroup_kernel(int mat_kind, bool damp) {
 }
 
 template <typename R>
-int Solver<R>::plan_groups(const mlx_mesh_desc* md) {
+int Solver<R>::plan_groups() {
   groups_ok = false;
+  groups_planned = true;
   const char* env = std::getenv("MLXPBD_GROUPS");
   const bool off = env && std::string(env) == "0", force = env && std::string(env) == "1";
   if (off || cluster_ok || persistent || T == 0) return MLX_OK;
-  // components (union-find over the tets' corners)
-  std::vector<int> parent(N);
-  for (int v = 0; v < N; ++v) parent[v] = v;
-  auto find = [&](int v) {
-    while (parent[v] != v) {
-      parent[v] = parent[parent[v]];
-      v = parent[v];
-    }
-    return v;
-  };
-  for (int e = 0; e < T; ++e) {
-    const int a = find(md->t[e] - 1);
-    for (int k = 1; k < 4; ++k) {
-      const int b = find(md->t[e + (size_t)k * T] - 1);
-      if (a != b) parent[std::max(a, b)] = std::min(a, b);
-    }
-  }
+  const std::vector<int>& root = comp_root;
   // component index of each vertex in order of first appearance; contiguous
   // vertex ranges means the index never decreases along the vertices
   std::vector<int> vcomp(N), cv0;
   {
     std::vector<int> label(N, -1);
     for (int v = 0; v < N; ++v) {
-      const int r = find(v);
+      const int r = root[v];
       if (label[r] < 0) {
         label[r] = (int)cv0.size();
         cv0.push_back(v);
@@ -1210,14 +1205,16 @@ int Solver<R>::plan_groups(const mlx_mesh_desc* md) {
   cv0.push_back(N);
   // tets of every (component, colour)
   std::vector<int> ccol((size_t)ncomp * C, 0), colcount(C, 0);
-  int lastc = 0;
-  for (int e = 0; e < T; ++e) {
-    const int c = vcomp[md->t[e] - 1];
-    if (c < lastc) return MLX_OK;  // elements are not grouped by component
-    lastc = c;
-    ++ccol[(size_t)c * C + md->element_color[e] - 1];
-    ++colcount[md->element_color[e] - 1];
+  std::vector<int> ecomp(T);  // component of every element
+  for (int q = 0; q < C; ++q) {
+    for (int s = color_off[q]; s < color_off[q + 1]; ++s) {
+      const int c = vcomp[vid_sorted[s].x];
+      ecomp[s2e[s]] = c;
+      ++ccol[(size_t)c * C + q];
+    }
+    colcount[q] = color_off[q + 1] - color_off[q];
   }
+  if (!std::is_sorted(ecomp.begin(), ecomp.end())) return MLX_OK;  // elements are not grouped by component
   int optin = 0, sms = 0;
   CU(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
   CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
@@ -1323,6 +1320,7 @@ int Solver<R>::plan_groups(const mlx_mesh_desc* md) {
   }
   if (best_cs == 0) return MLX_OK;
   if (!force && cs_force <= 0 && best.t >= t_colours) return MLX_OK;
+  if (flow_on && best_cs > 1) return MLX_OK;  // (k_layer_cgroups takes no contacts, what they are for then)
   const std::vector<int>& gv0 = best.gv0;
   const int G = (int)gv0.size() - 1;
   const int cs = best_cs;
@@ -1407,7 +1405,7 @@ int Solver<R>::launch_groups(const LayerStatic& ls, const int* dint, const mlx_s
                              const DevContacts& dc, const HostContactGroups* hc) {
   GroupArgs ga;
   ga.list = ls.identity_list ? nullptr : dint + ls.o_list;
-  ga.off = dint + ls.o_goff;
+  ga.off = ls.gr_off.template as<int>();
   ga.gv0 = d_gv0.as<int>();
   ga.tloc = d_tloc.as<int4>();
   ga.pin_off = d_gpin.as<int>();
@@ -1466,6 +1464,34 @@ int Solver<R>::launch_groups(const LayerStatic& ls, const int* dint, const mlx_s
                  : launch_group_kernel<R, 0>(&cfg, mat_kind, damp, td, ga, pos(), oldp, inv_h2, inv_h, dc, h, cr, pv, hg_);
   if (e != cudaSuccess) return set_error(MLX_ERR_CUDA, std::string("group layer launch: ") + cudaGetErrorString(e));
   return MLX_OK;
+}
+
+// Smallest vertex of every vertex's component (union-find over the tets'
+// corners in element order), for both plans below.
+template <typename R>
+void Solver<R>::find_components(const mlx_mesh_desc* md) {
+  if (!comp_root.empty()) return;
+  std::vector<int>& parent = comp_root;
+  parent.resize(N);
+  for (int v = 0; v < N; ++v) parent[v] = v;
+  auto find = [&](int v) {
+    while (parent[v] != v) {
+      parent[v] = parent[parent[v]];
+      v = parent[v];
+    }
+    return v;
+  };
+  for (int e = 0; e < T; ++e) {
+    int low = find(md->t[e] - 1);
+    for (int k = 1; k < 4; ++k) {
+      const int b = find(md->t[e + (size_t)k * T] - 1);
+      if (b == low) continue;
+      parent[std::max(low, b)] = std::min(low, b);
+      low = std::min(low, b);
+    }
+  }
+  // (a parent is never above its vertex, so one ascending pass reaches the roots)
+  for (int v = 0; v < N; ++v) parent[v] = parent[parent[v]];
 }
 
 // Shared memory and co-resident clusters of 1, 2, 4, 8 and 16 CTAs of k_flow.
@@ -1527,27 +1553,14 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
   if (!force && std::getenv("MLXPBD_GROUPS")) return MLX_OK;
   // components in element order; elements of one component that are not
   // consecutive make the whole mesh one component
-  std::vector<int> parent(N), comp_first;  // first element of every component
-  for (int v = 0; v < N; ++v) parent[v] = v;
-  auto find = [&](int v) {
-    while (parent[v] != v) {
-      parent[v] = parent[parent[v]];
-      v = parent[v];
-    }
-    return v;
-  };
-  for (int e = 0; e < T; ++e) {
-    const int a = find(md->t[e] - 1);
-    for (int k = 1; k < 4; ++k) {
-      const int b = find(md->t[e + (size_t)k * T] - 1);
-      if (a != b) parent[std::max(a, b)] = std::min(a, b);
-    }
-  }
+  find_components(md);
+  const std::vector<int>& root = comp_root;
+  std::vector<int> comp_first;  // first element of every component
   {
     std::vector<unsigned char> seen(N, 0);
     int last = -1;
     for (int e = 0; e < T; ++e) {
-      const int r = find(md->t[e] - 1);
+      const int r = root[md->t[e] - 1];
       if (r == last) continue;
       if (seen[r]) {
         comp_first.assign(1, 0);
@@ -1693,7 +1706,7 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
     const ushort4 q = eslot[s2e[s]];
     src[s] = make_ushort4(perm[q.x], perm[q.y], perm[q.z], perm[q.w]);
   }
-  CHECK(flow_tables());
+  CHECK(flow_tables(true));
   CU(cudaMemcpyAsync(fl_partd.p, fl_part.data(), sizeof(int) * (size_t)T, cudaMemcpyHostToDevice, stream));
   CU(cudaMemcpyAsync(fl_srcd.p, src.data(), sizeof(ushort4) * (size_t)T, cudaMemcpyHostToDevice, stream));
   CU(cudaStreamSynchronize(stream));
@@ -1707,13 +1720,13 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
 }
 
 template <typename R>
-int Solver<R>::flow_tables() {
+int Solver<R>::flow_tables(bool part_tables) {
   const size_t t = (size_t)T, n = (size_t)N;
   size_t used = 0;
   struct Part {
     DevPart* t;
     size_t bytes;
-  } parts[] = {{&fl_partd, sizeof(int) * t},       {&fl_srcd, sizeof(ushort4) * t},
+  } parts[] = {{&fl_partd, part_tables ? sizeof(int) * t : 0}, {&fl_srcd, part_tables ? sizeof(ushort4) * t : 0},
                {&ch_cor, sizeof(int) * 4 * t},     {&ch_off, sizeof(int) * (n + 1)},
                {&fl_at, sizeof(int) * (t + 4)},    {&fl_pin_at, pinned.empty() ? 0 : sizeof(int) * 3 * n},
                {&fl_mat, fl_iso ? sizeof(R) * 3 * t : 0}};
@@ -1770,7 +1783,7 @@ int Solver<R>::plan_sweep() {
   CU(cudaDeviceGetAttribute(&sw_sms, cudaDevAttrMultiProcessorCount, device));
   CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sweep_kernel(sizeof(R) == 8, mat_kind, damp), kSweepThreads, 0));
   if (per_sm < 1) return MLX_OK;
-  CHECK(flow_tables());
+  CHECK(flow_tables(false));
   CHECK(sw_rec.ensure(sizeof(SweepRec<R>) * (size_t)N));
   CHECK(sw_state.ensure(sizeof(SweepState)));
   CU(cudaMemsetAsync(sw_rec.p, 0, sizeof(SweepRec<R>) * (size_t)N, stream));
@@ -2227,6 +2240,46 @@ bool Solver<R>::statics_hit(const mlx_layer_desc* ld, const LayerWork& w) const 
   return true;
 }
 
+// (colour, group) ranges of a layer's elastic tets for the component-group
+// path: within a colour they are in element order, so each group's are one
+// range when the groups are ascending element ranges.
+template <typename R>
+int Solver<R>::build_groups(LayerStatic& ls) {
+  ls.gr_ok = false;
+  if (ls.nb > 0) return MLX_OK;  // (body-free layers only)
+  const int G = gr_G;
+  const int* list = ls.identity_list ? nullptr : ls.packed.data() + ls.o_list;
+  std::vector<int> goff((size_t)C * G + 1, 0);
+  int maxr = 0;
+  for (int c = 0; c < C; ++c) {
+    const int b = ls.identity_list ? color_off[c] : ls.color_start[c];
+    int last = -1;
+    for (int q = b; q < b + ls.color_count[c]; ++q) {
+      const int g = tgroup_sorted[list ? list[q] : q];
+      if (g < last) return MLX_OK;
+      last = g;
+      ++goff[(size_t)c * G + g + 1];
+    }
+  }
+  for (size_t q = 1; q < goff.size(); ++q) maxr = std::max(maxr, goff[q]);
+  // counts -> starts (in list positions, or sorted ids for the identity)
+  for (int c = 0; c < C; ++c) {
+    int run = ls.identity_list ? color_off[c] : ls.color_start[c];
+    for (int g = 0; g < G; ++g) {
+      const int cnt = goff[(size_t)c * G + g + 1];
+      goff[(size_t)c * G + g] = run;
+      run += cnt;
+    }
+  }
+  goff[(size_t)C * G] = ls.tets;
+  ls.gr_one = maxr <= gr_cs * kGroupThreads ? 1 : 0;
+  CHECK(ls.gr_off.ensure(sizeof(int) * goff.size()));
+  CU(cudaMemcpyAsync(ls.gr_off.p, goff.data(), sizeof(int) * goff.size(), cudaMemcpyHostToDevice, stream));
+  CU(cudaStreamSynchronize(stream));
+  ls.gr_ok = true;
+  return MLX_OK;
+}
+
 template <typename R>
 int Solver<R>::build_static(const mlx_layer_desc* ld, int col, LayerStatic& ls, bool capturing) {
   const uint8_t* isE = ld->is_elastic_element + (size_t)T * col;
@@ -2330,44 +2383,8 @@ int Solver<R>::build_static(const mlx_layer_desc* ld, int col, LayerStatic& ls, 
     ls.n_items = (int)(items.size() / kItemInts);
     ls.o_items = put(items);
   }
-  // (colour, group) ranges of the elastic tets for the component-group path:
-  // within a colour the elastic tets are in element order, so each group's
-  // are one range when the groups are ascending element ranges
   ls.gr_ok = false;
-  if (groups_ok) {
-    const int G = gr_G;
-    std::vector<int> goff((size_t)C * G + 1, 0);
-    bool mono = true;
-    int maxr = 0;
-    for (int c = 0; c < C && mono; ++c) {
-      const int b = ls.identity_list ? color_off[c] : ls.color_start[c];
-      const int n = ls.color_count[c];
-      int last = -1;
-      for (int q = 0; q < n; ++q) {
-        const int sidx = ls.identity_list ? b + q : list[b + q];
-        const int g = tgroup_sorted[sidx];
-        if (g < last) { mono = false; break; }
-        last = g;
-        ++goff[(size_t)c * G + g + 1];
-      }
-    }
-    if (mono) {
-      for (size_t q = 1; q < goff.size(); ++q) maxr = std::max(maxr, goff[q]);
-      // counts -> starts (in list positions, or sorted ids for the identity)
-      for (int c = 0; c < C; ++c) {
-        int run = ls.identity_list ? color_off[c] : ls.color_start[c];
-        for (int g = 0; g < G; ++g) {
-          const int cnt = goff[(size_t)c * G + g + 1];
-          goff[(size_t)c * G + g] = run;
-          run += cnt;
-        }
-      }
-      goff[(size_t)C * G] = ls.identity_list ? T : (int)list.size();
-      ls.gr_one = maxr <= gr_cs * kGroupThreads ? 1 : 0;
-      ls.o_goff = put(goff);
-      ls.gr_ok = true;
-    }
-  }
+  if (groups_ok) CHECK(build_groups(ls));
   ls.fl_ok = false;
   if (flow_on) CHECK(build_flow(ls, list));
   ls.sw_ok = false;
@@ -3952,6 +3969,12 @@ int Solver<R>::sim_set_obstacles(const mlx_obstacle* obs, int nobs, double resti
     CU(cudaMemcpyAsync(d_obs.p, o.data(), sizeof(Obstacle) * o.size(), cudaMemcpyHostToDevice, stream));
     CHECK(contact_colours());
     CU(cudaMemsetAsync(d_cscan.p, 0, sizeof(int) * (blocks_for(N, 256) + 2 + MLX_MAX_OBSTACLES), stream));
+    if (flow_on && !flow_forced && !groups_planned) {
+      CHECK(plan_groups());
+      std::vector<int>().swap(comp_root);
+      if (groups_ok)
+        for (auto& ls : sim_work.cache) CHECK(build_groups(*ls));
+    }
     CU(cudaStreamSynchronize(stream));
   }
   if (sim.graph) { cudaGraphExecDestroy(sim.graph); sim.graph = nullptr; }
