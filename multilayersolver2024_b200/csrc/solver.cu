@@ -357,6 +357,7 @@ struct LayerStatic {
   // dataflow path (flow.cuh): chunks of each part, corner words and slots
   bool fl_ok = false;
   int fl_chunks = 0, fl_max = 0;  // chunks, largest part's
+  int fl_planes_chunks = 0;       // chunks the planes have room for
   bool loose_pins = false;     // a pinned vertex has no elastic tet in this layer
   bool fl_loose_free = false;  // a vertex of no body has none
   bool fl_coloured = false;    // the corner words hold the contact phases
@@ -676,6 +677,7 @@ struct Solver final : SolverBase {
   // MLXPBD_PERSISTENT=1).
   bool flow_on = false;
   int fl_G = 0, fl_cs = 1, fl_slots = 0, fl_smem = 0;
+  int fl_chunks_all = 0;  // chunks of all tets: no layer has more
   std::vector<int> fl_part;                // [T] part of each sorted tet
   bool fl_reorder = false;                 // the parts are not runs of the element order
   // per mesh, in one allocation: part and corner slots of each sorted tet, the
@@ -1706,6 +1708,17 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
     const ushort4 q = eslot[s2e[s]];
     src[s] = make_ushort4(perm[q.x], perm[q.y], perm[q.z], perm[q.w]);
   }
+  {
+    const int P = fl_G * fl_cs;
+    std::vector<int> cnt(P);
+    for (int c = 0; c < C; ++c) {
+      std::fill(cnt.begin(), cnt.end(), 0);
+      for (int s = color_off[c]; s < color_off[c + 1]; ++s) ++cnt[fl_part[s]];
+      for (int n : cnt) fl_chunks_all += (n + 31) / 32;
+    }
+  }
+  // (shared by the layers of the host calls and of the resident stepper)
+  CHECK(fl_lam.ensure(sizeof(R) * 32 * (size_t)fl_chunks_all * (mat_kind == MAT_NH ? 2 : 6)));
   CHECK(flow_tables(true));
   CU(cudaMemcpyAsync(fl_partd.p, fl_part.data(), sizeof(int) * (size_t)T, cudaMemcpyHostToDevice, stream));
   CU(cudaMemcpyAsync(fl_srcd.p, src.data(), sizeof(ushort4) * (size_t)T, cudaMemcpyHostToDevice, stream));
@@ -1827,12 +1840,7 @@ int Solver<R>::link_sweep(LayerStatic& ls) {
   k_sweep_link<<<blocks_for(N, 128), 128, 0, stream>>>(ch_off.as<int>(), ch_cor.as<int>(), at, fl_pin_at.as<int>(), N,
                                                        ls.sw_corner.template as<unsigned short>(), at + T, at + T + 1, at + T + 2);
   CU(cudaGetLastError());
-  int* hs = h_scalar.as<int>();
-  CU(cudaMemcpyAsync(hs, at + T, sizeof(int) * 3, cudaMemcpyDeviceToHost, stream));
-  CU(cudaStreamSynchronize(stream));
-  ls.loose_pins = hs[0] != 0;
-  ls.sw_D = std::max(hs[1], 1);
-  ls.sw_vertices = std::max(hs[2], 1);
+  CU(cudaMemcpyAsync(h_scalar.p, at + T, sizeof(int) * 3, cudaMemcpyDeviceToHost, stream));  // (read by build_static)
   return MLX_OK;
 }
 
@@ -1938,18 +1946,13 @@ int Solver<R>::build_flow(LayerStatic& ls, const std::vector<int>& clist) {
       ch[0] = r.at + o;
       ch[1] = std::min(32, r.n - o) | r.c << 8;
     }
-  const size_t nq = (size_t)std::max(ls.fl_chunks, 1);
+  // The planes of a layer that changes from step to step: at its second size
+  // they take the mesh's, which no layer exceeds.
+  if (ls.fl_chunks > ls.fl_planes_chunks) ls.fl_planes_chunks = ls.fl_planes_chunks ? fl_chunks_all : ls.fl_chunks;
+  const size_t nq = (size_t)std::max(ls.fl_planes_chunks, 1);
   ls.o_fcorner = sizeof(R4<R>) * 32 * nq * flow_planes_of(flow_mat());
   ls.o_fvid = ls.o_fcorner + sizeof(uint4) * 64 * nq;
   CHECK(ls.fl_planes.ensure(ls.o_fvid + sizeof(int4) * 32 * nq));
-  // (the resident stepper's and the host calls' layers share the scratch:
-  // it only grows, and a grown one drops the recorded graphs)
-  const size_t lam = sizeof(R) * 32 * nq * (mat_kind == MAT_NH ? 2 : 6);
-  if (fl_lam.bytes < lam) {
-    drop_host_graph();
-    if (sim.graph) { cudaGraphExecDestroy(sim.graph); sim.graph = nullptr; }
-    CHECK(fl_lam.ensure(lam));
-  }
   ls.fl_ok = true;
   return MLX_OK;
 }
@@ -1982,9 +1985,7 @@ bool Solver<R>::sweep_pays(const LayerStatic& ls) const {
 // device.
 template <typename R>
 int Solver<R>::link_flow(LayerStatic& ls) {
-  ls.loose_pins = ls.fl_loose_free = false;
   ls.fl_coloured = d_vcc.p != nullptr;
-  CHECK(h_scalar.ensure(sizeof(double) * 8));
   int* at = fl_at.as<int>();
   int* dint = ls.dev.as<int>();
   int4* ch = reinterpret_cast<int4*>(dint + ls.o_fch);
@@ -2024,11 +2025,7 @@ int Solver<R>::link_flow(LayerStatic& ls) {
     void* args[] = {&td, &chc, &list, &m3, &rest, &vd};
     CU(cudaLaunchKernel(flow_pack_kernel(sizeof(R) == 8, flow_mat()), dim3(ls.fl_chunks), dim3(32), args, 0, stream));
   }
-  int* hs = h_scalar.as<int>();
-  CU(cudaMemcpyAsync(hs, at + T, sizeof(int) * 2, cudaMemcpyDeviceToHost, stream));
-  CU(cudaStreamSynchronize(stream));
-  ls.loose_pins = hs[0] != 0;
-  ls.fl_loose_free = hs[1] != 0;
+  CU(cudaMemcpyAsync(h_scalar.p, at + T, sizeof(int) * 3, cudaMemcpyDeviceToHost, stream));  // (read by build_static)
   return MLX_OK;
 }
 
@@ -2419,7 +2416,7 @@ int Solver<R>::build_static(const mlx_layer_desc* ld, int col, LayerStatic& ls, 
     ls.o_cllb = put(lb);
     CHECK(build_cluster_slots(ls, list));
   }
-  CHECK(ls.dev.ensure(sizeof(int) * ls.packed.size()));
+  CHECK(ls.dev.ensure(sizeof(int) * ls.packed.size(), ls.dev.p != nullptr));
   CHECK(ls.dev_rigid.ensure(N));
   CU(cudaMemcpyAsync(ls.dev.p, ls.packed.data(), sizeof(int) * ls.packed.size(), cudaMemcpyHostToDevice, stream));
   CU(cudaMemcpyAsync(ls.dev_rigid.p, isRV, N, cudaMemcpyHostToDevice, stream));
@@ -2428,6 +2425,13 @@ int Solver<R>::build_static(const mlx_layer_desc* ld, int col, LayerStatic& ls, 
   // the host copies above are pageable: make sure they finished before the
   // cached vectors can change
   CU(cudaStreamSynchronize(stream));
+  const int* found = h_scalar.as<int>();  // what link_flow or link_sweep found
+  ls.loose_pins = (ls.fl_ok || ls.sw_ok) && found[0] != 0;
+  ls.fl_loose_free = ls.fl_ok && found[1] != 0;
+  if (ls.sw_ok) {
+    ls.sw_D = std::max(found[1], 1);
+    ls.sw_vertices = std::max(found[2], 1);
+  }
   ls.valid = true;
   return MLX_OK;
 }
