@@ -39,10 +39,12 @@
 #include <cstdio>
 #include <cstring>
 #include <array>
+#include <future>
 #include <map>
 #include <memory>
 #include <mutex>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -705,7 +707,14 @@ struct Solver final : SolverBase {
   bool flow_keeps_coloured(const LayerStatic& ls) const {
     return flow_forced || sizeof(R) == 8 || ls.fl_max <= (mat_kind != MAT_NH && !(damp && mat_kind == MAT_STVK_BLOCKS) ? 110 : 700);
   }
-  int plan_flow(const mlx_mesh_desc* md);
+  // what cut_flow leaves for plan_flow: 0 neither, 1 dataflow, 2 through L2
+  struct FlowCut {
+    int rc = MLX_OK, path = 0;
+    std::string error;
+    std::vector<ushort4> src;  // slots of every sorted tet's corners
+  };
+  int cut_flow(const mlx_mesh_desc* md, FlowCut& cut);
+  int plan_flow(const FlowCut& cut);
   int upload_pin_at();
   int build_flow(LayerStatic& ls, const std::vector<int>& list);
   int link_flow(LayerStatic& ls);
@@ -925,6 +934,23 @@ int Solver<R>::create(const mlx_mesh_desc* md) {
     }
   }
 
+  // The plan's host part (5 ms for 98 k tets, most of it the breadth-first cut)
+  // runs beside the packing and the copies (7 ms); in place for small meshes,
+  // where a thread costs more than the plan.
+  FlowCut cut;
+  auto cut_now = [&]() {
+    cut.rc = cut_flow(md, cut);
+    if (cut.rc != MLX_OK) cut.error = g_err;  // (the message is the thread's own)
+  };
+  std::future<void> cutting;
+  if (T >= 4096) {
+    try {
+      cutting = std::async(std::launch::async, cut_now);
+    } catch (const std::system_error&) {  // no thread to be had
+    }
+  }
+  if (!cutting.valid()) cut_now();
+
   // ---- host-side packing of the rest data in sorted order ----
   const int stride = mat_stride(mat_kind);
   std::vector<int4> vid(T);
@@ -1026,7 +1052,8 @@ int Solver<R>::create(const mlx_mesh_desc* md) {
   if (cluster_ok) vowner = mp.vowner;
   // (beside the dataflow sweeps the groups take contacts only: planned with
   // the first obstacles)
-  CHECK(plan_flow(md));
+  if (cutting.valid()) cutting.get();
+  CHECK(plan_flow(cut));
   if (!flow_on && !sweep_on && !flow_forced) {
     find_components(md);
     CHECK(plan_groups());
@@ -1543,15 +1570,18 @@ static int flow_limits(int device, bool fp64, int mat, bool damp, int threads, F
   return MLX_OK;
 }
 
-// Plan of the dataflow path: how many groups of whole components, on clusters
-// of how many CTAs, and the part of every element.
+// Plan of the dataflow path, the host's part: how many groups of whole
+// components, on clusters of how many CTAs, and the part of every element.
 template <typename R>
-int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
+int Solver<R>::cut_flow(const mlx_mesh_desc* md, FlowCut& cut) {
   const char* env = std::getenv("MLXPBD_FLOW");
   const bool force = env && std::string(env) == "1";
   flow_forced = force || (env && std::string(env) == "2");
   if ((env && std::string(env) == "0") || persistent || cluster_ok || std::getenv("MLXPBD_PDL")) return MLX_OK;
-  if (env && std::string(env) == "2") return plan_sweep();
+  if (env && std::string(env) == "2") {
+    cut.path = 2;
+    return MLX_OK;
+  }
   if (!force && std::getenv("MLXPBD_GROUPS")) return MLX_OK;
   // components in element order; elements of one component that are not
   // consecutive make the whole mesh one component
@@ -1576,7 +1606,12 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
   const int ncomp = (int)comp_first.size();
   comp_first.push_back(T);
   FlowLimits lim;
-  CHECK(flow_limits(device, sizeof(R) == 8, flow_mat(), damp, flow_threads<R>(), lim));
+  {
+    // (whether the blocks are isotropic is not known yet: the same limits)
+    DeviceGuard g(device);
+    CHECK(flow_limits(device, sizeof(R) == 8, mat_kind == MAT_STVK_BLOCKS && !damp ? (int)MAT_STVK_ISO : mat_kind, damp,
+                      flow_threads<R>(), lim));
+  }
   fl_smem = lim.smem;
   int want_cs = 0;
   if (const char* q = std::getenv("MLXPBD_FLOW_CS")) want_cs = std::atoi(q);
@@ -1667,7 +1702,10 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
     best = pl;
     break;
   }
-  if (best.t < 0) return force || t_l2 > t_colours ? MLX_OK : plan_sweep();
+  if (best.t < 0) {
+    cut.path = force || t_l2 > t_colours ? 0 : 2;
+    return MLX_OK;
+  }
   if (best.cs > 1 && best.sum > 3 * (long long)N / 2) {
     // parts that share many vertices (an element order of thin slabs): cut
     // the breadth-first order instead where that shares fewer
@@ -1685,7 +1723,7 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
       order.clear();
     }
   }
-  flow_on = true;
+  cut.path = 1;
   fl_reorder = !order.empty();
   fl_G = best.G;
   fl_cs = best.cs;
@@ -1702,7 +1740,8 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
   for (int p = 0; p < fl_G * fl_cs; ++p)
     for (int i = best.first[p]; i < best.first[p + 1]; ++i) epart[order.empty() ? i : order[i]] = p;
   fl_part.resize(T);
-  std::vector<ushort4> src(T);
+  std::vector<ushort4>& src = cut.src;
+  src.resize(T);
   for (int s = 0; s < T; ++s) {
     fl_part[s] = epart[s2e[s]];
     const ushort4 q = eslot[s2e[s]];
@@ -1717,11 +1756,23 @@ int Solver<R>::plan_flow(const mlx_mesh_desc* md) {
       for (int n : cnt) fl_chunks_all += (n + 31) / 32;
     }
   }
+  return MLX_OK;
+}
+
+// The device's part of the plan.
+template <typename R>
+int Solver<R>::plan_flow(const FlowCut& cut) {
+  if (cut.rc != MLX_OK) return set_error(cut.rc, cut.error);
+  if (cut.path == 0) return MLX_OK;
+  if (cut.path == 2) return plan_sweep();
+  FlowLimits lim;  // (sets the kernel up)
+  CHECK(flow_limits(device, sizeof(R) == 8, flow_mat(), damp, flow_threads<R>(), lim));
+  flow_on = true;
   // (shared by the layers of the host calls and of the resident stepper)
   CHECK(fl_lam.ensure(sizeof(R) * 32 * (size_t)fl_chunks_all * (mat_kind == MAT_NH ? 2 : 6)));
   CHECK(flow_tables(true));
   CU(cudaMemcpyAsync(fl_partd.p, fl_part.data(), sizeof(int) * (size_t)T, cudaMemcpyHostToDevice, stream));
-  CU(cudaMemcpyAsync(fl_srcd.p, src.data(), sizeof(ushort4) * (size_t)T, cudaMemcpyHostToDevice, stream));
+  CU(cudaMemcpyAsync(fl_srcd.p, cut.src.data(), sizeof(ushort4) * (size_t)T, cudaMemcpyHostToDevice, stream));
   CU(cudaStreamSynchronize(stream));
   if (fl_iso) {
     const int rows[3] = {0, 1, 9};  // alpha's diagonal, off-diagonal and shear entries
