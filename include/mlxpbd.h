@@ -348,6 +348,10 @@ int mlx_wait_probe(int32_t device, int32_t kind, int64_t limit_ns, int32_t* time
  * after the iteration that found it, whatever its stop rules -- and the calls
  * after it are not affected. */
 int mlx_sweep_wait_probe(mlx_solver* solver);
+/* Diagnostic of the sweeps through L2: sets the counter their vertex tags
+ * start from (at most 2^32 - 2^29 - 1, where the next launch clears the
+ * records and starts over).  MLX_ERR_UNSUPPORTED where the solver has none. */
+int mlx_sweep_tags_probe(mlx_solver* solver, uint32_t base);
 
 /* xpbdLayer3D.buildLayers (3d/integrator/xpbdLayer3D.m:601-619) followed by
  * xpbdLayer2D.findBoundaryVertices (2d/integrator/xpbdLayer2D.m:551-569) on

@@ -162,6 +162,7 @@ SIGNATURES = {
     "mlx_pcg_solve": ([C.c_void_p, C.c_double, _f64p, C.c_int32, _f64p, _f64p], C.c_int),
     "mlx_wait_probe": ([C.c_int32, C.c_int32, C.c_int64, C.POINTER(C.c_int32)], C.c_int),
     "mlx_sweep_wait_probe": ([C.c_void_p], C.c_int),
+    "mlx_sweep_tags_probe": ([C.c_void_p, C.c_uint32], C.c_int),
     "mlx_build_layers": ([C.c_void_p, _f64p, _f64p, C.c_double, C.c_int32, _i32p, _f64p, _f64p, C.c_int32, _u8p,
                           _i32p, _i32p, _u8p, _u8p, _u8p, _i32p], C.c_int),
     "mlx_mlp_create": ([C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_uint64, C.c_int32,

@@ -736,7 +736,9 @@ struct Solver final : SolverBase {
   int build_sweep(LayerStatic& ls);
   int link_sweep(LayerStatic& ls);
   bool sweep_layer(const LayerStatic& ls, int iterations) const {
-    return sweep_on && ls.sw_ok && ls.tile.empty() && (long long)ls.sw_D * std::max(iterations, 1) < kSweepMaxTags;
+    // (neither the tags of a launch nor a CTA's count of its chunks, sweep.cuh, may run out)
+    return sweep_on && ls.sw_ok && ls.tile.empty() && (long long)ls.sw_D * std::max(iterations, 1) < kSweepMaxTags &&
+           (long long)(ls.sw_chunks / std::max(sw_sms, 1) + 1) * iterations < (1ll << 31);
   }
   int launch_sweep(const LayerStatic& ls, const int* dint, R h, int iterations, bool pins);
   int build_cluster_slots(LayerStatic& ls, const std::vector<int>& list);
@@ -748,6 +750,14 @@ struct Solver final : SolverBase {
   int begin_sweeps();
   int sweep_wait_probe() override {
     probe_sweep_wait = true;
+    return MLX_OK;
+  }
+  int sweep_tags_probe(uint32_t base) override {
+    DeviceGuard g(device);
+    if (!sweep_on) return set_error(MLX_ERR_UNSUPPORTED, "the solver has no sweeps through L2");
+    const unsigned b = std::min<unsigned>(base, 0u - (unsigned)(2 * kSweepMaxTags) - 1);
+    CU(cudaMemcpyAsync(sw_state.p, &b, sizeof(unsigned), cudaMemcpyHostToDevice, stream));
+    CU(cudaStreamSynchronize(stream));
     return MLX_OK;
   }
   bool probe_sweep_wait = false;  // the next call starts as if a sweep's wait had run out
@@ -5101,6 +5111,12 @@ int mlx_pcg_solve(mlx_solver* s, double h, const double* b, int32_t iterations, 
   return mlx::guarded([&]() -> int {
     if (!s) return set_error(MLX_ERR_ARGUMENT, "null solver");
     return s->impl->pcg_solve(h, b, iterations, x, resvec);
+  });
+}
+int mlx_sweep_tags_probe(mlx_solver* s, uint32_t base) {
+  return mlx::guarded([&]() -> int {
+    if (!s) return set_error(MLX_ERR_ARGUMENT, "null solver");
+    return s->impl->sweep_tags_probe(base);
   });
 }
 int mlx_sweep_wait_probe(mlx_solver* s) {

@@ -52,6 +52,7 @@ struct SolverBase {
   virtual int sim_set_obstacles(const mlx_obstacle* obs, int nobs, double restitution) = 0;
   virtual int sim_contact_count(int32_t* n) = 0;
   virtual int sweep_wait_probe() = 0;
+  virtual int sweep_tags_probe(uint32_t base) = 0;
   virtual int sim_monitor(double* ra, int cap, int32_t* len, int32_t* total_it, double* run_until,
                           int32_t* status) = 0;
   virtual int ws_configure(int record, int mode, mlx_mlp* net, double gate, const float* fmean, const float* fstd,
