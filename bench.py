@@ -601,9 +601,10 @@ def run_ours(args, rank, world, local):
             sweep_kernel = "k_layer_cluster (whole projectGS loop of a layer)"
         elif solver_launch_path.startswith("dataflow"):
             sweep_kernel = ("k_flow (body-free layers: the whole projectGS loop in one launch, vertex records in shared "
-                            "memory; layers with bodies: one launch per sweep)")
+                            "memory; layers with bodies: one launch per sweep, where colour launches are not shorter)")
         elif solver_launch_path.startswith("version-ordered"):
-            sweep_kernel = "k_sweep (all colours of a sweep in one launch, vertex records through L2)"
+            sweep_kernel = ("k_sweep (all colours of a sweep in one launch, vertex records through L2; monitored loops "
+                            "k_project_color where that is shorter)")
         elif "CTAs each owning whole components" in solver_launch_path:
             sweep_kernel = ("k_layer_groups (whole projectGS loop of each body-free layer; algorithmic bytes without "
                             "vertex records, which stay in shared memory) + k_project_color (layers with bodies)")
@@ -651,8 +652,8 @@ def run_ours(args, rank, world, local):
             iters_le = fleg["iterations_per_step"]
             per_iter = fixed_launches / max(sum(sc.iterations), 1)
             launches = int(sum(it * (per_iter + 2) for it in iters_le))
-            launch_note = ("estimate: iterations of the timed steps x (launches per fixed-count iteration + the "
-                           "monitor's 2)")
+            launch_note = ("estimate, a lower one where the monitored loop takes a launch per colour: iterations of "
+                           "the timed steps x (launches per fixed-count iteration + the monitor's 2)")
             if to_res["value_leg"] == "learned_pcg":
                 # each Newton-PCG correction: 7 launches + 2 per PCG iteration, one before the fine layer
                 # and one after every `every` of its iterations (the fine layer holds most iterations)

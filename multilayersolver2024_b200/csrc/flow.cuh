@@ -33,14 +33,15 @@
 // What bounds it: a vertex's chain, one projection (~1,200 cycles for a
 // Neo-Hookean tet), its stores' way to the next CTA and the wake-up per tet,
 // ~0.9 us per colour on meshes whose chunks leave the SMs idle; above ~100
-// chunks per CTA the warps share the SM (~250 cycles per chunk).  A colour
-// launch costs ~1.9 us whatever its size.  Per sweep (B200, Neo-Hookean FP32,
-// this path / colour launches): 27,648 tets on 16 CTAs 29 / 58 us, 98,304
-// tets 41 / 58 us, 64 scenes of 866 k tets 53 / 95 us.  Polling the records'
-// versions instead of mbarriers measured 33 us on the 27,648 tets (the polls
-// take the shared-memory pipe from the projections), st.async inside the CTA
-// too 45 us on the 98,304 (it goes out to the network and back), the rest data
-// gathered per tet instead of read from chunk planes 58 us on the 98,304.
+// chunks per CTA the warps share the SM (~250 cycles per chunk).  Whole
+// recorded steps, us per sweep of this path / colour launches (B200,
+// Neo-Hookean FP32): 27,648 tets on 16 CTAs 33 / 61, 98,304 tets 43 / 68;
+// other sizes, materials and precisions: sweep_times.h.  Variants, the sweeps
+// alone: polling the records' versions instead of mbarriers 33 us against 29 on
+// the 27,648 tets (the polls take the shared-memory pipe from the
+// projections), st.async inside the CTA too 45 against 41 on the 98,304 (it
+// goes out to the network and back), the rest data gathered per tet instead of
+// read from chunk planes 58 against 41 there.
 // Bulk copies of the rest data into shared memory and prefetches of the next
 // chunk's lines into L1 or L2 gave nothing, two or four smaller CTAs per SM
 // neither.

@@ -643,13 +643,14 @@ struct Solver final : SolverBase {
   // Chosen at mlx_create when the components are contiguous vertex and tet
   // ranges, every group fits in a CTA's shared memory and the estimated sweep
   // is shorter than with colour launches; MLXPBD_GROUPS=0 turns it off, =1
-  // skips the estimate.  Beside the dataflow sweeps they keep the body-free
-  // layers with device-detected contacts in the reference's order (after every
-  // sweep): a thread per contact here, while there a vertex's contact holds up
-  // its tets' next sweep.  Resting boxes, 4 steps here / there: 6 of 750 tets
-  // 3.2 / 3.4 ms, 32 of 3,072 3.8 / 4.9, 32 of 10,368 5.6 / 5.9 (with few
-  // contacts 5.5 / 5.0); contacts coloured with the tets 3.9 / 3.2, 5.2 / 4.2,
-  // 7.9 / 5.3, and without contacts 70 / 39 us per sweep of the largest.
+  // skips the estimate.  Beside the dataflow sweeps they are planned with the
+  // first obstacles and keep the body-free layers with device-detected contacts
+  // in the reference's order (after every sweep): a thread per contact here,
+  // while there a vertex's contact holds up its tets' next sweep, by as much as
+  // vertices are in contact, which only the device knows.  Resting boxes, 4
+  // steps here / there: 6 of 750 tets 3.2 / 3.4 ms, 32 of 3,072 3.8 / 4.9, 32
+  // of 10,368 5.6 / 5.9 (with few contacts 5.5 / 5.0); contacts coloured with
+  // the tets 3.9 / 3.2, 5.2 / 4.2, 7.9 / 5.3 (more: flow_keeps_coloured).
   bool groups_ok = false;
   int gr_G = 0;
   int gr_cs = 1;  // CTAs per group (a thread-block cluster when > 1)
@@ -673,10 +674,11 @@ struct Solver final : SolverBase {
   int launch_groups(const LayerStatic& ls, const int* dint, const mlx_solve_params* P, int iterations,
                     const DevContacts& dc, const HostContactGroups* hc = nullptr);
   // Dataflow path (flow.cuh): the sweeps of a layer in one launch, ordered by
-  // vertex versions.  Default where its estimate is the shortest;
-  // MLXPBD_FLOW=0 turns it off and =1 skips the estimate, and naming another
-  // launch path does too (MLXPBD_GROUPS, MLXPBD_PDL, MLXPBD_CLUSTER=1,
-  // MLXPBD_PERSISTENT=1).
+  // vertex versions.  Default where its estimate (sweep_times.h) is the
+  // shortest, per mesh for the fixed loop of all tets and per layer for one
+  // iteration per launch and for contacts; MLXPBD_FLOW=0 turns it off, =1
+  // skips the estimates, and naming another launch path turns it off too
+  // (MLXPBD_GROUPS, MLXPBD_PDL, MLXPBD_CLUSTER=1, MLXPBD_PERSISTENT=1).
   bool flow_on = false;
   int fl_G = 0, fl_cs = 1, fl_slots = 0, fl_smem = 0;
   int fl_chunks_all = 0;  // chunks of all tets: no layer has more
@@ -726,9 +728,9 @@ struct Solver final : SolverBase {
   int launch_flow(const LayerStatic& ls, const int* dint, const mlx_solve_params* P, int iterations, bool pins,
                   const DevContacts& dc, int after);
   // The sweeps of a layer in one launch over the whole GPU, versions through
-  // L2 (sweep.cuh): components too large for the dataflow path's clusters.
-  // MLXPBD_FLOW=0 and the other switches above turn it off too,
-  // MLXPBD_FLOW=2 skips the estimate.
+  // L2 (sweep.cuh): FP32 components of about 0.2 to 1.3 M tets, which would keep
+  // one cluster busy longer.  MLXPBD_FLOW=0 and the other switches above turn
+  // it off too, MLXPBD_FLOW=2 skips the estimates.
   bool sweep_on = false;
   int sw_sms = 0;
   DevBuf sw_rec, sw_minv, sw_state;
@@ -1924,7 +1926,7 @@ int Solver<R>::launch_sweep(const LayerStatic& ls, const int* dint, R h, int ite
   a.N = N;
   a.pins = pins && !pinned.empty() ? 1 : 0;
   // a colour's chunks per CTA: one waiting chunk at a time while a CTA has
-  // few (98 k tets: 55 us per sweep with one, 59 with two), two above that
+  // few (98 k tets, sweeps alone: 55 us with one, 59 with two), two above that
   // (393 k: 65 and 63); 866 k tets want eight warps (75 us; 106 with four)
   const double per = (double)ls.sw_chunks / ((double)C * sw_sms);
   a.gate = per < 2 ? 1 : 2;

@@ -32,12 +32,15 @@
 // ends the launch.
 //
 // What bounds it: the chain of a vertex, one projection (~1,200 cycles) and
-// one way through L2 (~2,000 cycles under load) per colour.  For components
-// that the clusters of flow.cuh cannot hold or that would keep 16 SMs busy
-// longer: 393,216 Neo-Hookean tets in FP32 take 62 us per sweep here, 85 with
-// a launch per colour, 112 on one cluster; 98,304 tets 53, 58 and 41 us.
-// Measured and not used: chunks of 16 tets (81 us on the 393,216), records
-// padded to a sector or a line (62 to 72 us), a pause between polls (+2 us).
+// one way through L2 (~2,000 cycles under load) per tet.  For components that
+// would keep one cluster of flow.cuh busy longer: 393,216 Neo-Hookean tets in
+// FP32 take 75 us per sweep of a fixed loop here, 96 with a launch per colour,
+// 138 on one cluster; one iteration per launch (a monitored loop, its monitor
+// included) 97, 96 and 172, so that takes the colour launches; FP64 147, 128
+// and 201 (three words a record), so FP64 does not come here.  Above 1.3 M tets
+// the records and rest data leave L2 (3.5 M: 290, colours 218).  Variants on
+// the 393,216, the sweeps alone (62 us): chunks of 16 tets 81, records padded
+// to a sector or a line 62 to 72, a pause between polls +2.
 #pragma once
 
 #include "common.cuh"

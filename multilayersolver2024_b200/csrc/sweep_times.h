@@ -47,7 +47,7 @@ inline const SweepTimes& sweep_times(bool fp64, SweepMat m) {
                                       {1.30, 0.17, 0.60, 2.50, 5.5e-5, 3.45}},
                                      {{1.10, 0.215, 0.30, 2.10, 1.15e-4, 4.8},
                                       {1.56, 0.28, 0.62, 2.65, 1.4e-4, 5.4},
-                                      {2.30, 0.37, 0.65, 3.35, 1.4e-4, 6.6},
+                                      {2.30, 0.37, 0.65, 3.35, 1.2e-4, 6.6},
                                       {1.58, 0.27, 0.60, 2.90, 1.1e-4, 5.7},
                                       {1.88, 0.34, 0.60, 3.25, 9.0e-5, 6.4}}};
   return t[fp64 ? 1 : 0][m];
