@@ -276,7 +276,7 @@ inline const void* flow_pack_kernel(bool fp64, int mat_kind) {
 }
 // k_flow of a precision and material (flow_fp32.cu, flow_fp64.cu); `ct`: with
 // device-detected contacts, `small`: at most 256 threads (FP32: twice the
-// registers, none spilled).
+// registers, none spilled; StVK with contacts always so).
 const void* flow_kernel_fp32(int mat_kind, bool damp, bool ct, bool small);
 const void* flow_kernel_fp64(int mat_kind, bool damp, bool ct);
 inline const void* flow_kernel(bool fp64, int mat_kind, bool damp, bool ct, bool small) {

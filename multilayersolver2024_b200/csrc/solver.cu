@@ -703,11 +703,11 @@ struct Solver final : SolverBase {
   bool sweep_pays(const LayerStatic& ls) const;
   // Coloured contacts of a body-free layer that the component groups could
   // take.  Resting blocks, us per sweep here / there, by chunks of the largest
-  // part: FP32 StVK 20 45/54, 81 48/87, 140 118/92, 166 105/90, 875 470/302;
-  // Neo-Hookean 140 87/84, 648 252/251, 875 338/278; damped 166 131/136.  FP64
-  // is never longer here (875: 394/391).
+  // part: FP32 StVK 20 45/54, 81 48/87, 177 98/91 (no contact yet 74/74), 906
+  // 417/302; Neo-Hookean 177 77/85, 906 333/278; damped 178 105/136.  FP64 is
+  // never longer here (906: 394/391).
   bool flow_keeps_coloured(const LayerStatic& ls) const {
-    return flow_forced || sizeof(R) == 8 || ls.fl_max <= (mat_kind != MAT_NH && !(damp && mat_kind == MAT_STVK_BLOCKS) ? 110 : 700);
+    return flow_forced || sizeof(R) == 8 || ls.fl_max <= (mat_kind != MAT_NH && !(damp && mat_kind == MAT_STVK_BLOCKS) ? 200 : 700);
   }
   // what cut_flow leaves for plan_flow: 0 neither, 1 dataflow, 2 through L2
   struct FlowCut {
@@ -2009,11 +2009,14 @@ int Solver<R>::build_flow(LayerStatic& ls, const std::vector<int>& clist) {
       ch[0] = r.at + o;
       ch[1] = std::min(32, r.n - o) | r.c << 8;
     }
-  // The planes of a layer that changes from step to step: at its second size
-  // they take the mesh's, which no layer exceeds.
-  if (ls.fl_chunks > ls.fl_planes_chunks) ls.fl_planes_chunks = ls.fl_planes_chunks ? fl_chunks_all : ls.fl_chunks;
+  // The planes of a layer that may change from step to step take the mesh's
+  // size, which no layer exceeds: from the start up to 64 MB, at the layer's
+  // second size above.
+  const size_t rest = sizeof(R4<R>) * 32 * flow_planes_of(flow_mat());
+  if (ls.fl_chunks > ls.fl_planes_chunks)
+    ls.fl_planes_chunks = ls.fl_planes_chunks || fl_chunks_all * (rest + 96 * 16) <= (size_t(64) << 20) ? fl_chunks_all : ls.fl_chunks;
   const size_t nq = (size_t)std::max(ls.fl_planes_chunks, 1);
-  ls.o_fcorner = sizeof(R4<R>) * 32 * nq * flow_planes_of(flow_mat());
+  ls.o_fcorner = rest * nq;
   ls.o_fvid = ls.o_fcorner + sizeof(uint4) * 64 * nq;
   CHECK(ls.fl_planes.ensure(ls.o_fvid + sizeof(int4) * 32 * nq));
   ls.fl_ok = true;
@@ -2125,8 +2128,14 @@ int Solver<R>::launch_flow(const LayerStatic& ls, const int* dint, const mlx_sol
   // Eight warps with all the registers they want where a CTA has up to four
   // chunks per colour (us for 10 sweeps and a step's rest, 512 -> 256 threads:
   // 32 boxes of 10,368 tets on 4 CTAs each 411 -> 387, 48,384 tets on 16 CTAs
-  // 375 -> 359), sixteen above (98,304 tets 447 -> 498).
-  const bool small = ls.fl_max <= 4 * C;
+  // 375 -> 359), sixteen above (98,304 tets 447 -> 498); the other materials
+  // cross there too (us per sweep, 512 / 256 threads, 36 k tets StVK 36.1 / 34.3,
+  // damped 58.8 / 52.5, 98 k 43.8 / 51.6 and 69.2 / 70.7).  With contacts, whose
+  // code spills at 128 registers, eight warps but for very large Neo-Hookean
+  // parts (resting blocks, chunks of the largest part: 87 Neo-Hookean 74 / 48,
+  // damped 116 / 63; 177 86 / 76 and 146 / 115; 340 100 / 97 and 172 / 130; 664
+  // Neo-Hookean 252 / 292; 906 333 / 356, StVK 463 / 417).
+  const bool small = after != 0 ? mat_kind != MAT_NH || ls.fl_max <= 400 : ls.fl_max <= 4 * C;
   cfg.blockDim = dim3(32 * std::min((small ? 256 : flow_threads<R>()) / 32, ls.fl_max));
   cfg.dynamicSmemBytes = (size_t)fl_slots * sizeof(R4<R>) + 8 * (size_t)ls.fl_max;
   cfg.stream = stream;

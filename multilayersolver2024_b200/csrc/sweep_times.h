@@ -40,22 +40,23 @@ struct SweepTimes {
 enum SweepMat : int { SWEEP_NH, SWEEP_BLOCKS, SWEEP_BLOCKS_DAMPED, SWEEP_LAME, SWEEP_LAME_DAMPED };
 
 inline const SweepTimes& sweep_times(bool fp64, SweepMat m) {
-  static const SweepTimes t[2][5] = {{{0.98, 0.137, 0.36, 1.80, 5.0e-5, 2.85},
-                                      {0.98, 0.137, 0.50, 1.92, 7.5e-5, 2.85},
-                                      {1.50, 0.21, 0.70, 2.30, 6.5e-5, 3.8},
-                                      {1.07, 0.145, 0.55, 2.27, 5.5e-5, 3.0},
-                                      {1.30, 0.17, 0.60, 2.50, 5.5e-5, 3.45}},
-                                     {{1.10, 0.215, 0.30, 2.10, 1.15e-4, 4.8},
-                                      {1.56, 0.28, 0.62, 2.65, 1.4e-4, 5.4},
-                                      {2.30, 0.37, 0.65, 3.35, 1.2e-4, 6.6},
-                                      {1.58, 0.27, 0.60, 2.90, 1.1e-4, 5.7},
-                                      {1.88, 0.34, 0.60, 3.25, 9.0e-5, 6.4}}};
+  static const SweepTimes t[2][5] = {{{0.98, 0.137, 0.27, 1.80, 5.0e-5, 2.85},
+                                      {0.98, 0.137, 0.33, 1.92, 7.5e-5, 2.85},
+                                      {1.50, 0.21, 0.36, 2.30, 6.5e-5, 3.8},
+                                      {1.07, 0.145, 0.33, 2.27, 5.5e-5, 3.0},
+                                      {1.30, 0.17, 0.33, 2.50, 5.5e-5, 3.45}},
+                                     {{1.10, 0.215, 0.26, 2.10, 1.15e-4, 4.8},
+                                      {1.56, 0.28, 0.45, 2.65, 1.4e-4, 5.4},
+                                      {2.30, 0.37, 0.56, 3.35, 1.2e-4, 6.6},
+                                      {1.58, 0.27, 0.45, 2.90, 1.1e-4, 5.7},
+                                      {1.88, 0.34, 0.48, 3.25, 9.0e-5, 6.4}}};
   return t[fp64 ? 1 : 0][m];
 }
 
 // The dataflow sweep of `colours` colours whose largest part has `chunks`
 // chunks, on `ctas` CTAs.  A chunk takes longer where most SMs are busy: 83 k
-// tets per 16 CTAs, 1 / 4 clusters 40 / 45 us FP32, 92 / 131 damped FP64.
+// tets per 16 CTAs, 1 / 4 clusters 40 / 45 us FP32, 92 / 131 damped FP64; with
+// resting contacts 0.25 / 0.36 us a chunk on 16 / 72 CTAs (FP32 Neo-Hookean).
 // once: one iteration per launch, which reads positions and multipliers anew
 // (FP64, 20 / 140 / 875 chunks of 148 CTAs: 18 of 50, 32 of 97, 419 of 717).
 inline double flow_us(const SweepTimes& t, bool fp64, SweepMat m, double colours, double chunks, int ctas, bool once,
@@ -63,7 +64,7 @@ inline double flow_us(const SweepTimes& t, bool fp64, SweepMat m, double colours
   const double busy = std::min(1.0, ctas / 148.0);
   const double shared = 1.0 + 0.9 * std::max(0.0, busy - 0.25);
   const double chain = t.chain * colours + (contacts ? 17.0 : 0.0);
-  const double issue = chunks * (contacts ? t.contact * std::max(1.0, shared / 1.36) : t.chunk * shared);
+  const double issue = chunks * (contacts ? t.contact * (1.0 + 1.3 * std::clamp(busy - 0.1, 0.0, 0.35)) : t.chunk * shared);
   const double q = std::max(0.0, chunks - 0.5 * colours);  // (half a chunk per colour is rounding)
   const double again = fp64 ? 6.0 + q * (0.12 + busy * (0.15 + 0.00035 * q))
                             : m == SWEEP_NH ? 5.0 + q * (0.04 + 0.08 * busy) : 8.0 + q * (0.07 + 0.08 * busy);

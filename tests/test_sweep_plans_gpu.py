@@ -78,6 +78,26 @@ def test_elements_not_grouped_by_component(gpu, monkeypatch, path, dims, copies)
         np.testing.assert_array_equal(x, y)
 
 
+@pytest.mark.parametrize("energy", [NH, STVK])
+@pytest.mark.parametrize("coloring", [False, True])
+def test_contacts_of_a_large_part(gpu, monkeypatch, energy, coloring):
+    """More than 400 chunks of 32 tets in one CTA."""
+    out = []
+    for flag in ("0", "1"):
+        monkeypatch.setenv("MLXPBD_FLOW", flag)
+        monkeypatch.setenv("MLXPBD_GROUPS", "0")
+        monkeypatch.setenv("MLXPBD_FLOW_CS", "1")
+        s, sim = _sim(_blocks((20, 12, 12), 1, energy=energy), coloring=coloring, v0z=-1.0)
+        sim.set_obstacles([PlaneContactFinder3D([0.0, 0.0, 1.0], [0.0, 0.0, 0.001])])
+        sim.step(3)
+        assert sim.contact_count() > 0
+        assert s.launch_path.startswith("dataflow") == (flag == "1")
+        out.append(sim.state())
+        s.close()
+    for x, y in zip(*out):
+        np.testing.assert_array_equal(x, y)
+
+
 @pytest.mark.parametrize("energy,prec", [(NH, _lib.MLX_FP32), (STVK, _lib.MLX_FP32), (NH, _lib.MLX_FP64)])
 @pytest.mark.parametrize("path", ["1", "2"])
 def test_layers_that_grow(gpu, monkeypatch, energy, prec, path):
