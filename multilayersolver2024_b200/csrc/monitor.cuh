@@ -73,10 +73,10 @@ __global__ void k_mon_loop_begin(MonState* ms, cudaGraphConditionalHandle loop, 
 // simpleMonitorError's rules (xpbdLayer3D.m:515-544), then the loop test.
 // With ns_every > 0 it also sets `ns`, the condition of the Newton-PCG
 // correction (pcg.cuh) that closes the iteration: after every ns_every
-// iterations of the last layer, when the loop goes on.  `sweep_error`: set by
-// a sweep whose wait ran out.
+// iterations of the last layer, when the loop goes on.  `sweep_failed`: the
+// wait of a sweep ran out.
 __device__ __forceinline__ void mon_iter_end(MonState* ms, cudaGraphConditionalHandle loop, int iterations,
-                                             int is_last, const MonParams& mp, const int* sweep_error,
+                                             int is_last, const MonParams& mp, int sweep_failed,
                                              cudaGraphConditionalHandle ns = 0, int ns_every = 0) {
   ms->it += 1;
   ms->total_iterations += 1;
@@ -106,7 +106,7 @@ __device__ __forceinline__ void mon_iter_end(MonState* ms, cudaGraphConditionalH
     ms->error = 1;
     ms->end_layer = 1;
   }
-  if (__ldcg(sweep_error) != 0) {
+  if (sweep_failed) {
     ms->error = 3;
     ms->stop = 1;
   }
@@ -118,7 +118,7 @@ __device__ __forceinline__ void mon_iter_end(MonState* ms, cudaGraphConditionalH
 
 __global__ void k_mon_iter_end(MonState* ms, cudaGraphConditionalHandle loop, int iterations, int is_last,
                                MonParams mp, const int* sweep_error, cudaGraphConditionalHandle ns, int ns_every) {
-  mon_iter_end(ms, loop, iterations, is_last, mp, sweep_error, ns, ns_every);
+  mon_iter_end(ms, loop, iterations, is_last, mp, *sweep_error, ns, ns_every);
 }
 
 }  // namespace mlx

@@ -525,7 +525,8 @@ struct Solver final : SolverBase {
     cudaGraphExec_t graph = nullptr;
     long long launches_per_step = 0;
   } sim;
-  DevBuf d_vel, d_pin_mask, d_gsync;
+  DevBuf d_vel, d_pin_mask;
+  DevPart d_gsync, h_gsync;  // parts of d_scalar and h_scalar
   // obstacles of the resident stepper (contacts detected on the device)
   std::vector<Obstacle> sim_obs;
   double sim_restitution = 1e-2;
@@ -609,7 +610,6 @@ struct Solver final : SolverBase {
                     double* normals, double* points, double* comp, int32_t* K) override;
   int sim_set_obstacles(const mlx_obstacle* obs, int nobs, double restitution) override;
   int sim_contact_count(int32_t* n) override;
-  PinnedBuf h_gsync;
   PinnedBuf h_mon;  // the device monitor's state, staged for a layer solve replayed as a graph
   long long last_launches = 0;
   // Layers that neither the dataflow sweeps nor the sweeps through L2 (below)
@@ -763,6 +763,7 @@ struct Solver final : SolverBase {
     return MLX_OK;
   }
   bool probe_sweep_wait = false;  // the next call starts as if a sweep's wait had run out
+  bool sweep_flag_clear = true;   // the last call ended with the flag read as 0
   cudaLaunchConfig_t pdl_config(int grid, int block) const {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
@@ -1032,13 +1033,14 @@ int Solver<R>::create(const mlx_mesh_desc* md) {
   CHECK(d_ri.ensure(sizeof(double4) * N));
   CHECK(d_s2e.ensure(sizeof(int) * T));
   CHECK(d_partials.ensure(sizeof(double) * 1024));
-  CHECK(d_scalar.ensure(sizeof(double) * 8));  // [0] residual, [1] norm of resv, [7] k_residual_monitor's ticket
-  CU(cudaMemsetAsync(d_scalar.p, 0, sizeof(double) * 8, stream));
-  CHECK(h_scalar.ensure(sizeof(double) * 8));
-  // [0..3] grid barrier of the persistent kernel, [4] error flag of the dataflow path
-  CHECK(d_gsync.ensure(sizeof(unsigned int) * 8));
-  CHECK(h_gsync.ensure(sizeof(int) * 8));
-  CU(cudaMemsetAsync(d_gsync.p, 0, sizeof(unsigned int) * 8, stream));
+  // [0] residual, [1] norm of resv, [7] k_residual_monitor's ticket; behind
+  // them, so that one copy brings both, gsync: [0..3] grid barrier of the
+  // persistent kernel, [4] error flag of the one-launch sweeps
+  CHECK(d_scalar.ensure(sizeof(double) * 8 + sizeof(int) * 8));
+  CU(cudaMemsetAsync(d_scalar.p, 0, sizeof(double) * 8 + sizeof(int) * 8, stream));
+  CHECK(h_scalar.ensure(sizeof(double) * 8 + sizeof(int) * 8));
+  d_gsync.p = d_scalar.as<char>() + sizeof(double) * 8;
+  h_gsync.p = h_scalar.as<char>() + sizeof(double) * 8;
   {
     const char* q = std::getenv("MLXPBD_PDL");
     pdl = !(q && std::string(q) == "0");
@@ -2602,9 +2604,8 @@ int Solver<R>::residual(const ContactData& cd, double contact_resistance, double
   if (dc && dc->nobs) CHECK(contact_residual_partials(*dc, contact_resistance, h, partials + tetBlocks + cBlocks, &dBlocks));
   k_finish_norm<256><<<1, 256, 0, stream>>>(partials, tetBlocks + cBlocks + dBlocks, d_scalar.as<double>());
   CU(cudaGetLastError());
-  CU(cudaMemcpyAsync(h_scalar.p, d_scalar.p, sizeof(double), cudaMemcpyDeviceToHost, stream));
-  if (flow_on || sweep_on)
-    CU(cudaMemcpyAsync(h_gsync.p, d_gsync.p, sizeof(unsigned int) * 8, cudaMemcpyDeviceToHost, stream));
+  // (with the flags of the sweeps behind it)
+  CU(cudaMemcpyAsync(h_scalar.p, d_scalar.p, sizeof(double) * 8 + sizeof(int) * 8, cudaMemcpyDeviceToHost, stream));
   CU(cudaStreamSynchronize(stream));
   *out = h_scalar.as<double>()[0];
   return MLX_OK;
@@ -2722,6 +2723,8 @@ __global__ void __launch_bounds__(256) k_residual_monitor(TetData<R> td, const R
                                                           cudaGraphConditionalHandle ns, int ns_every) {
   pdl_launch_dependents();
   pdl_wait();
+  // (volatile: loaded here, not on the last thread's way to the loop's condition)
+  const int failed = *reinterpret_cast<const volatile int*>(sweep_error);
   double acc[1] = {residual_tets<R, MAT>(td, pos, inv_h2, inv_h, inv_h2_d, blockIdx.x * blockDim.x + threadIdx.x,
                                          gridDim.x * blockDim.x)};
   block_sum<1>(acc);
@@ -2740,7 +2743,7 @@ __global__ void __launch_bounds__(256) k_residual_monitor(TetData<R> td, const R
   if (threadIdx.x == 0) {
     ms->res = sqrt(sum[0]);
     *ticket = 0;
-    mon_iter_end(ms, loop, iterations, is_last, mp, sweep_error, ns, ns_every);
+    mon_iter_end(ms, loop, iterations, is_last, mp, failed, ns, ns_every);
   }
 }
 
@@ -3287,8 +3290,9 @@ int Solver<R>::reset_gsync() {
 // whatever the one before it ended with.
 template <typename R>
 int Solver<R>::begin_sweeps() {
-  CU(cudaMemsetAsync(sweep_error(), probe_sweep_wait ? 1 : 0, sizeof(int), stream));
-  probe_sweep_wait = false;
+  if (!sweep_flag_clear || probe_sweep_wait)
+    CU(cudaMemsetAsync(sweep_error(), probe_sweep_wait ? 1 : 0, sizeof(int), stream));
+  probe_sweep_wait = sweep_flag_clear = false;
   return MLX_OK;
 }
 
@@ -3687,6 +3691,7 @@ int Solver<R>::layer_solve(const mlx_layer_desc* ld, const mlx_solve_params* P, 
   CU(cudaStreamSynchronize(stream));
   cpack_used = 0;  // no copy of the contact lists is in flight now
   CHECK(check_gsync());
+  sweep_flag_clear = true;
   if (P->compute_residuals && replayed) {
     // replayed with the stop rules on the device
     const MonState* hm = h_mon.as<MonState>();
@@ -4846,7 +4851,10 @@ int Solver<R>::sim_step(int nsteps, int use_graph, double* device_ms) {
     cudaEventDestroy(e1);
   }
   CU(cudaStreamSynchronize(stream));
-  if (nsteps > 0) CHECK(check_gsync());
+  if (nsteps > 0) {
+    CHECK(check_gsync());
+    sweep_flag_clear = true;
+  }
   return MLX_OK;
 }
 
