@@ -2723,8 +2723,11 @@ __global__ void __launch_bounds__(256) k_residual_monitor(TetData<R> td, const R
                                                           cudaGraphConditionalHandle ns, int ns_every) {
   pdl_launch_dependents();
   pdl_wait();
-  // (volatile: loaded here, not on the last thread's way to the loop's condition)
-  const int failed = *reinterpret_cast<const volatile int*>(sweep_error);
+  // (volatile: loaded here, not on the last thread's way to the loop's
+  // condition; by the one thread of a CTA that may need it, or 4,700 warps ask
+  // one L2 slice)
+  int failed = 0;
+  if (threadIdx.x == 0) failed = *reinterpret_cast<const volatile int*>(sweep_error);
   double acc[1] = {residual_tets<R, MAT>(td, pos, inv_h2, inv_h, inv_h2_d, blockIdx.x * blockDim.x + threadIdx.x,
                                          gridDim.x * blockDim.x)};
   block_sum<1>(acc);
@@ -3119,7 +3122,9 @@ int Solver<R>::run_layers(const mlx_layer_desc* ld, const mlx_solve_params* P, c
         cudaLaunchConfig_t cfg = pdl_config(tb, 256);
         cudaLaunchAttribute attr = pdl_attr();
         cfg.attrs = &attr;
-        cfg.numAttrs = pdl ? 1 : 0;
+        // (behind colour launches its early CTAs take room from the last of them:
+        // 831 k tets FP64 192 us per iteration with, 186 without)
+        cfg.numAttrs = pdl && (flow || sweep) ? 1 : 0;
         const R4<R>* pc = pos();
         const double ihd = 1.0 / (h * h);
         const int* serr = sweep_error();
