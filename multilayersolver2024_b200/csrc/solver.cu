@@ -659,6 +659,7 @@ struct Solver final : SolverBase {
   DevBuf d_gv0, d_tloc, d_gpin;
   int plan_groups();
   bool groups_planned = false;
+  int group_cs = 0;  // MLXPBD_GROUP_CS
   std::vector<int> comp_root;
   void find_components(const mlx_mesh_desc* md);
   int build_groups(LayerStatic& ls);
@@ -1046,6 +1047,7 @@ int Solver<R>::create(const mlx_mesh_desc* md) {
     pdl = !(q && std::string(q) == "0");
     const char* hgv = std::getenv("MLXPBD_HOST_GRAPH");
     host_graph_on = !(hgv && std::string(hgv) == "0");
+    if (const char* gc = std::getenv("MLXPBD_GROUP_CS")) group_cs = std::atoi(gc);
     const char* n = std::getenv("MLXPBD_PERSIST_CTAS");
     int sms = 0;
     CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
@@ -1225,7 +1227,9 @@ template <typename R>
 int Solver<R>::plan_groups() {
   groups_ok = false;
   groups_planned = true;
-  const char* env = std::getenv("MLXPBD_GROUPS");
+  // (the switches are read when the solver is created: beside the dataflow
+  // sweeps, planned later, they were not set)
+  const char* env = flow_on ? nullptr : std::getenv("MLXPBD_GROUPS");
   const bool off = env && std::string(env) == "0", force = env && std::string(env) == "1";
   if (off || cluster_ok || persistent || T == 0) return MLX_OK;
   const std::vector<int>& root = comp_root;
@@ -1347,12 +1351,10 @@ int Solver<R>::plan_groups() {
   double t_colours = 0;
   for (int q = 0; q < C; ++q)
     if (colcount[q]) t_colours += 2.6 + (double)colcount[q] * (double)bytes_per_tet() / 6.5e6;
-  int cs_force = 0;
-  if (const char* f = std::getenv("MLXPBD_GROUP_CS")) cs_force = std::atoi(f);
   Plan best;
   int best_cs = 0;
   for (int cs : {1, 2, 4, 8}) {
-    if (cs_force > 0 && cs != cs_force) continue;
+    if (group_cs > 0 && cs != group_cs) continue;
     Plan pl;
     const double t = form(cs, pl);
     if (t < 0) continue;
@@ -1362,7 +1364,7 @@ int Solver<R>::plan_groups() {
     }
   }
   if (best_cs == 0) return MLX_OK;
-  if (!force && cs_force <= 0 && best.t >= t_colours) return MLX_OK;
+  if (!force && group_cs <= 0 && best.t >= t_colours) return MLX_OK;
   if (flow_on && best_cs > 1) return MLX_OK;  // (k_layer_cgroups takes no contacts, what they are for then)
   const std::vector<int>& gv0 = best.gv0;
   const int G = (int)gv0.size() - 1;
